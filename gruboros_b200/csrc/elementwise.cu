@@ -452,6 +452,23 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16
   }
 }
 
+// a *= *scale in place (bf16, fp32 product); a scale of exactly 1 leaves without touching `a`.
+__global__ void scale_bf16_kernel(__nv_bfloat16* __restrict__ a, int64_t n, const float* __restrict__ scale) {
+  const float s = *scale;
+  if (s == 1.f) return;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 8; i += stride) {
+    uint4 v = reinterpret_cast<uint4*>(a)[i];
+    v.x = pack_bf16(bf16_lo(v.x) * s, bf16_hi(v.x) * s);
+    v.y = pack_bf16(bf16_lo(v.y) * s, bf16_hi(v.y) * s);
+    v.z = pack_bf16(bf16_lo(v.z) * s, bf16_hi(v.z) * s);
+    v.w = pack_bf16(bf16_lo(v.w) * s, bf16_hi(v.w) * s);
+    reinterpret_cast<uint4*>(a)[i] = v;
+  }
+  if (blockIdx.x == 0)
+    for (int64_t i = n / 8 * 8 + threadIdx.x; i < n; i += blockDim.x) a[i] = __float2bfloat16(__bfloat162float(a[i]) * s);
+}
+
 static int num_sms() {
   static int n = 0;
   if (!n) {
@@ -582,5 +599,13 @@ extern "C" int grb_cast_f32_bf16(const float* in, void* out, int64_t n, void* st
   const int64_t threads = (n + 7) / 8;
   cast_f32_bf16_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, ST(stream)>>>(
       in, reinterpret_cast<__nv_bfloat16*>(out), n);
+  return LAUNCH_OK();
+}
+
+extern "C" int grb_scale_bf16(void* a, int64_t n, const float* scale, void* stream) {
+  if (n == 0) return 0;
+  if (reinterpret_cast<uintptr_t>(a) & 15) return -2;
+  const int blocks = static_cast<int>(std::min<int64_t>((n / 8 + 255) / 256 + 1, num_sms() * 4));
+  scale_bf16_kernel<<<blocks, 256, 0, ST(stream)>>>(reinterpret_cast<__nv_bfloat16*>(a), n, scale);
   return LAUNCH_OK();
 }

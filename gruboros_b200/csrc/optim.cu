@@ -28,9 +28,12 @@ __device__ __forceinline__ void sf_update(float g, float& y, float& z, float& v,
   z = z - a.lr * gh;
 }
 
+// `dyn` (nullable): the step's scalars in device memory instead of the launch arguments, so that a recorded pass can
+// be replayed with the values of another step.
 __global__ void __launch_bounds__(256)
 sfadamw_kernel(float* __restrict__ y, float* __restrict__ z, float* __restrict__ v, float* __restrict__ g,
-               __nv_bfloat16* __restrict__ w16, int64_t n, SfArgs a, int zero_grad) {
+               __nv_bfloat16* __restrict__ w16, int64_t n, SfArgs a, const SfArgs* __restrict__ dyn, int zero_grad) {
+  if (dyn) a = *dyn;
   const int64_t nvec = n / 4;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec; i += stride) {
@@ -262,7 +265,29 @@ extern "C" int grb_sfadamw_step(float* y, float* z, float* v, float* g, void* w1
   if (w16 && (reinterpret_cast<uintptr_t>(w16) & 7)) return -2;
   SfArgs a{lr, beta1, beta2, bias2, eps, wd, ckp1, gscale};
   sfadamw_kernel<<<grid_for(n / 4), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      y, z, v, g, reinterpret_cast<__nv_bfloat16*>(w16), n, a, zero_grad);
+      y, z, v, g, reinterpret_cast<__nv_bfloat16*>(w16), n, a, nullptr, zero_grad);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+namespace grb {
+__global__ void sf_hyper_kernel(SfArgs* dst, SfArgs a) { *dst = a; }
+}  // namespace grb
+
+extern "C" int grb_sf_hyper(float* dst, float lr, float beta1, float beta2, float bias2, float eps, float wd, float ckp1,
+                            float gscale, void* stream) {
+  sf_hyper_kernel<<<1, 1, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<SfArgs*>(dst),
+                                                                        SfArgs{lr, beta1, beta2, bias2, eps, wd, ckp1, gscale});
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+extern "C" int grb_sfadamw_dyn_step(float* y, float* z, float* v, float* g, void* w16, int64_t n, const float* hyper,
+                                    int zero_grad, void* stream) {
+  if (n <= 0) return 0;
+  if (((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(v) |
+        reinterpret_cast<uintptr_t>(g)) & 15) || (reinterpret_cast<uintptr_t>(w16) & 7) || !hyper)
+    return -2;
+  sfadamw_kernel<<<grid_for(n / 4), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      y, z, v, g, reinterpret_cast<__nv_bfloat16*>(w16), n, SfArgs{}, reinterpret_cast<const SfArgs*>(hyper), zero_grad);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

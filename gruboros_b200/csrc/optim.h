@@ -10,6 +10,12 @@ extern "C" {
 // w16 (optional) receives bf16(y); zero_grad != 0 clears g in the same pass.
 int grb_sfadamw_step(float* y, float* z, float* v, float* g, void* w16, int64_t n, float lr, float beta1, float beta2,
                      float bias2, float eps, float wd, float ckp1, float gscale, int zero_grad, void* stream);
+// The same step with its scalars read from `hyper` (8 floats in device memory, written by grb_sf_hyper on the stream):
+// a recorded launch can then be replayed for every step.
+int grb_sf_hyper(float* dst, float lr, float beta1, float beta2, float bias2, float eps, float wd, float ckp1, float gscale,
+                 void* stream);
+int grb_sfadamw_dyn_step(float* y, float* z, float* v, float* g, void* w16, int64_t n, const float* hyper, int zero_grad,
+                         void* stream);
 // Sharded variant: this rank owns flat elements [begin, begin+count) (multiples of 4); y, g are full flat buffers,
 // z, v hold the shard only; bf16(y) is stored into all `world` mirrors w16_peers[r] (peer pointers).
 int grb_sfadamw_shard_step(float* y, float* z, float* v, float* g, void* const* w16_peers, int world, int64_t begin,

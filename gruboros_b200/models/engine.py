@@ -35,6 +35,7 @@ import torch
 
 from ..ops import kernels as K
 from ..ops import _lib as L
+from ..ops.graph import Recorder
 from ..utils.flat import FlatParams, lookup
 
 NUM_SMS_DEFAULT = 148
@@ -100,6 +101,8 @@ class _Buffers:
         self.xwf = e(M, D)
         self.ssqf = e(M, P, dtype=f32)
         self.rstdf = e(M, dtype=f32)
+        self.tokens = e(B, T + 1, dtype=torch.uint8)   # input of a recorded pass
+        self.recorder = Recorder()
         self.labels = e(M, dtype=torch.uint8)
         self.loss_rows = e(M, dtype=f32)
         self.loss = torch.zeros(1, dtype=f32, device=dev)
@@ -238,24 +241,64 @@ class FusedEngine:
             raise ValueError(f"expected {self.depth} hidden states, got {len(prev)}")
         if any(p.numel() == 0 for p in prev):
             return False                      # empty carry: same as no carry
+        n = bufs.B * self.Di
         for i, p in enumerate(prev):
-            if p.numel() != bufs.B * self.Di:
+            if p.numel() != n:
                 raise ValueError(f"hidden state {i} has {p.numel()} elements, expected batch {bufs.B} x inner dim {self.Di}")
-        bufs.h0.copy_(torch.stack([p.reshape(bufs.B, self.Di) for p in prev]))
+        p0 = prev[0]
+        base = p0.data_ptr()
+        if (p0.dtype == torch.float32 and p0.device == bufs.h0.device
+                and all(p.dtype == torch.float32 and p.is_contiguous() and p.data_ptr() == base + 4 * n * i for i, p in enumerate(prev))
+                and p0.storage_offset() + n * self.depth <= p0.untyped_storage().nbytes() // 4
+                and all(p.untyped_storage().data_ptr() == p0.untyped_storage().data_ptr() for p in prev)):
+            # the states of one earlier pass, as _hiddens_out returns them: consecutive views, one copy
+            bufs.h0.copy_(p0.detach().as_strided(bufs.h0.shape, bufs.h0.stride()))
+        else:
+            bufs.h0.copy_(torch.stack([p.reshape(bufs.B, self.Di) for p in prev]))
         return True
 
     # -------------------------------------------------------------- forward
+    def _recordable(self) -> bool:
+        """Whether a pass is the same launches over the same buffers every time, so that it can be replayed: one replica
+        with all its parameters resident (sharded storage and peer gradients change addresses between passes)."""
+        return self.store is None and self.grad_sink is None and self.param_gather is None and not self.nvtx
+
+    def _key(self, *what):
+        f = self.flat
+        return (*what, f.data.data_ptr(), f.grad.data_ptr(), f.w16.data_ptr(), K.GEMM_MODE, self.wgrad_split)
+
+    def _begin(self, tokens: torch.Tensor, T: int, prev_hiddens, train: bool) -> _Buffers:
+        """What precedes the launches of a forward pass: current bf16 weights, the buffer set, the carried state."""
+        self.ensure_flat(tokens.device)
+        self.sync_weights()
+        bufs = self.buffers(tokens.shape[0], T, train)
+        has_h0 = self._load_carry(bufs, prev_hiddens)
+        if self._recordable():
+            if not has_h0:
+                bufs.h0.zero_()          # "no state" is a state of zeros: one recording serves both
+            has_h0 = True
+            n = min(tokens.shape[1], T + 1)
+            bufs.tokens[:, :n].copy_(tokens[:, :n])
+        bufs.h0_valid = has_h0
+        return bufs
+
     def _forward(self, tokens: torch.Tensor, T: int, prev_hiddens, *, train: bool, want_loss: bool, alpha: float = 1.0):
         """tokens: uint8 [B, >=T(+1)] on the device.  Returns the buffer set holding the results."""
-        dev = tokens.device
-        self.ensure_flat(dev)
-        self.sync_weights()
-        B = tokens.shape[0]
-        bufs = self.buffers(B, T, train)
+        bufs = self._begin(tokens, T, prev_hiddens, train)
         n0 = K.LAUNCHES
+        if self._recordable():
+            bufs.recorder.run(self._key("forward", want_loss, alpha),
+                              lambda: self._launch_forward(bufs, bufs.tokens, want_loss, alpha), tokens.device)
+        else:
+            self._launch_forward(bufs, tokens, want_loss, alpha)
+        self._gen += 1
+        bufs.gen = self._gen
+        self.launches_last = K.LAUNCHES - n0
+        return bufs
+
+    def _launch_forward(self, bufs: _Buffers, tokens: torch.Tensor, want_loss: bool, alpha: float) -> None:
+        B, T, train, has_h0 = bufs.B, bufs.T, bufs.train, bufs.h0_valid
         M, D, Di, Fh, V = bufs.M, self.D, self.Di, self.F, self.V
-        has_h0 = self._load_carry(bufs, prev_hiddens)
-        bufs.h0_valid = has_h0
         ix = self._idx
         pg = self.param_gather
         if pg is not None:
@@ -297,10 +340,6 @@ class FusedEngine:
         else:
             K.linear_fwd(bufs.xwf, self._w(ix["logits"]), bufs.logits, epi=K.EPI_STORE_F32,
                          rownorm=(bufs.ssqf, D, eps, None))
-        self._gen += 1
-        bufs.gen = self._gen
-        self.launches_last = K.LAUNCHES - n0
-        return bufs
 
     # ------------------------------------------------------------- backward
     def unit_ranges(self):
@@ -317,11 +356,22 @@ class FusedEngine:
     def _backward(self, bufs: _Buffers, unit_done=None) -> None:
         """Gradients of the last training forward on `bufs`, accumulated into the flat fp32 gradient buffer.
         `unit_done(j)` is called as soon as every gradient of unit j (see unit_ranges) has been launched."""
+        self._check_backward(bufs)
+        n0 = K.LAUNCHES
+        if unit_done is None and self._recordable():
+            bufs.recorder.run(self._key("backward"), lambda: self._launch_backward(bufs), self.device)
+        else:
+            self._launch_backward(bufs, unit_done)
+        self._gen += 1          # activations are consumed
+        self.launches_last += K.LAUNCHES - n0
+
+    def _check_backward(self, bufs: _Buffers) -> None:
         if not bufs.train or bufs.gen != self._gen:
             raise RuntimeError("backward must follow the training forward whose activations it uses")
-        n0 = K.LAUNCHES
         if self.grad_sink is None and self.store is None:
             self.flat.reclaim_discarded_grads()     # gradients the caller dropped (p.grad = None) start from zero
+
+    def _launch_backward(self, bufs: _Buffers, unit_done=None) -> None:
         B, T, M = bufs.B, bufs.T, bufs.M
         D, Di, Fh, V = self.D, self.Di, self.F, self.V
         ix = self._idx
@@ -375,8 +425,6 @@ class FusedEngine:
         self._wgrad(bufs.onehot, bufs.dres16, ix["emb"], sk(V, D))
         if unit_done is not None:
             unit_done(self.depth + 1)
-        self._gen += 1          # activations are consumed
-        self.launches_last += K.LAUNCHES - n0
 
     # ----------------------------------------------------------- public API
     @staticmethod
@@ -406,23 +454,49 @@ class FusedEngine:
         """
         tokens = self._as_tokens(chunk)
         T = tokens.shape[1] - 1
-        bufs = self._forward(tokens, T, prev_hiddens, train=True, want_loss=True, alpha=loss_scale)
         if stepper is None and optimizer is not None:
+            self.ensure_flat(tokens.device)
             stepper = _LocalStepper(optimizer, self.flat)
-        if stepper is None:
-            self._backward(bufs)
+        if isinstance(stepper, _LocalStepper) and self._recordable():
+            bufs = self._train_pass(tokens, T, prev_hiddens, loss_scale, stepper)
         else:
-            units = self.unit_ranges()
-            main = torch.cuda.current_stream()
-            if self._side is None:
-                self._side = torch.cuda.Stream(device=self.device)
-            side = self._side
-            stepper.begin(units)
-            self._backward(bufs, lambda j: stepper.unit_done(j, main, side))
-            stepper.end(main, side)
+            bufs = self._forward(tokens, T, prev_hiddens, train=True, want_loss=True, alpha=loss_scale)
+            if stepper is None:
+                self._backward(bufs)
+            else:
+                main, side = torch.cuda.current_stream(), self._side_stream()
+                stepper.begin(self.unit_ranges())
+                self._backward(bufs, lambda j: stepper.unit_done(j, main, side))
+                stepper.end(main, side)
         if self.store is None:
             self.flat.attach_grads()
         return bufs.loss[0].clone(), self._hiddens_out(bufs)
+
+    def _side_stream(self):
+        if self._side is None:
+            self._side = torch.cuda.Stream(device=self.device)
+        return self._side
+
+    def _train_pass(self, tokens, T, prev_hiddens, alpha, stepper) -> _Buffers:
+        """Forward, backward and the folded optimizer step as one recorded pass (the step's scalars are in device memory)."""
+        bufs = self._begin(tokens, T, prev_hiddens, True)
+        n0 = K.LAUNCHES
+        self._gen += 1
+        bufs.gen = self._gen
+        self._check_backward(bufs)
+        stepper.begin(self.unit_ranges())
+
+        def body():
+            self._launch_forward(bufs, bufs.tokens, True, alpha)
+            main, side = torch.cuda.current_stream(), self._side_stream()
+            self._launch_backward(bufs, lambda j: stepper.unit_done(j, main, side))
+            stepper.join(main, side)
+
+        bufs.recorder.run(self._key("train", alpha, *stepper.addresses()), body, self.device)
+        stepper.finish()
+        self._gen += 1          # activations are consumed
+        self.launches_last = K.LAUNCHES - n0
+        return bufs
 
     def decoder(self, batch: int = 1, use_graph: bool = True, impl: str = "tc"):
         """Token-by-token generation state for `batch` sequences (``models/decode.py``), cached per configuration."""
@@ -465,18 +539,28 @@ class _LocalStepper:
 
     def begin(self, units):
         self.units = units
-        self.hp = self.optimizer.begin_ranged_step(self.flat)
+        self.hyper = self.optimizer.begin_ranged_step(self.flat)
+
+    def addresses(self):
+        """Device addresses that the launches of unit_done depend on beside the flat parameters."""
+        return self.hyper.data_ptr(), self.flat.sf_z.data_ptr(), self.flat.sf_v.data_ptr()
 
     def unit_done(self, j, main, side):
         ev = torch.cuda.Event()
         ev.record(main)
         with torch.cuda.stream(side):
             side.wait_event(ev)
-            self.optimizer.step_range(self.flat, self.units[j][0], self.units[j][1], self.hp)
+            self.optimizer.step_range(self.flat, self.units[j][0], self.units[j][1], self.hyper)
+
+    def join(self, main, side):
+        main.wait_stream(side)
+
+    def finish(self):
+        self.optimizer.end_ranged_step(self.flat)
 
     def end(self, main, side):
-        main.wait_stream(side)
-        self.optimizer.end_ranged_step(self.flat)
+        self.join(main, side)
+        self.finish()
 
 
 class _FusedLoss(torch.autograd.Function):
@@ -493,7 +577,7 @@ class _FusedLoss(torch.autograd.Function):
     def backward(ctx, gloss):
         engine, bufs = ctx.engine, ctx.bufs
         # d logits were written for d(loss) = 1; fold the incoming scale in (device-side, no sync)
-        bufs.dlogits.copy_(bufs.dlogits.float() * gloss)
+        K.scale_bf16(bufs.dlogits, gloss.detach().float().contiguous())
         engine._backward(bufs)
         if engine.store is None:
             engine.flat.attach_grads()

@@ -78,6 +78,14 @@ _SIGS = {
     "grb_decode_tc": [_I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P],
     "grb_decode_gemv": [_I, _P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _I, _I, _P, _P],
     "grb_sfadamw_step": [_P, _P, _P, _P, _P, _L, _F, _F, _F, _F, _F, _F, _F, _F, _I, _P],
+    "grb_sf_hyper": [_P, _F, _F, _F, _F, _F, _F, _F, _F, _P],
+    "grb_sfadamw_dyn_step": [_P, _P, _P, _P, _P, _L, _P, _I, _P],
+    "grb_scale_bf16": [_P, _L, _P, _P],
+    "grb_capture_begin": [_P],
+    "grb_capture_end": [_P, C.POINTER(C.c_void_p)],
+    "grb_graph_launch": [_P, _P],
+    "grb_graph_destroy": [_P],
+    "grb_is_capturing": [_P],
     "grb_merge": [_P, _P, _F, _P, _P, _F, _P, _P, _F, _P, _L, _P],
 }
 

@@ -271,6 +271,25 @@ def sfadamw_step(y, z, v, g, w16, *, lr, beta1, beta2, bias2, eps, wd, ckp1, gsc
     _count()
 
 
+def sf_hyper(dst, *, lr, beta1, beta2, bias2, eps, wd, ckp1, gscale=1.0):
+    """Write a step's scalars into ``dst`` (fp32 [8] on the device), where ``sfadamw_dyn_step`` reads them."""
+    L.check(L.lib().grb_sf_hyper(dst.data_ptr(), lr, beta1, beta2, bias2, eps, wd, ckp1, gscale, L.stream()), "grb_sf_hyper")
+    _count()
+
+
+def sfadamw_dyn_step(y, z, v, g, w16, hyper, zero_grad=True):
+    """``sfadamw_step`` with its scalars in device memory (see ``sf_hyper``)."""
+    L.check(L.lib().grb_sfadamw_dyn_step(y.data_ptr(), z.data_ptr(), v.data_ptr(), g.data_ptr(), L.ptr(w16), y.numel(),
+                                         hyper.data_ptr(), int(zero_grad), L.stream()), "grb_sfadamw_dyn_step")
+    _count()
+
+
+def scale_bf16(a, scale):
+    """a *= scale in place; ``scale`` is an fp32 tensor of one element on the device."""
+    L.check(L.lib().grb_scale_bf16(a.data_ptr(), a.numel(), scale.data_ptr(), L.stream()), "grb_scale_bf16")
+    _count()
+
+
 def merge(pairs, w16, n):
     """pairs: up to three (dst_tensor, src_ptr_or_tensor, alpha); dst = (1-alpha) dst + alpha src, fused bf16 recast."""
     args = []

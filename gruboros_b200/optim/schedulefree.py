@@ -219,20 +219,27 @@ class AdamWScheduleFree(Optimizer):
                 and all(lookup(p) is owner for p in self.param_groups[0]["params"][:1]))
 
     @torch.no_grad()
-    def begin_ranged_step(self, owner) -> dict:
+    def begin_ranged_step(self, owner) -> torch.Tensor:
+        """Advance the step's bookkeeping and put its scalars into device memory (returned: fp32 [8]), from where the
+        ranges' kernels read them - the launches themselves are the same for every step and can be recorded."""
         group = self.param_groups[0]
         if not group["train_mode"]:
             raise RuntimeError("Optimizer was not in train mode when step is called. Call .train() first.")
         self._init_state(group)
         self._adopt_flat_state(group)
-        return self._advance(group)
+        from ..ops import kernels as K
+        hyper = getattr(owner, "sf_hyper", None)
+        if hyper is None:
+            hyper = owner.sf_hyper = torch.empty(8, dtype=torch.float32, device=owner.device)
+        K.sf_hyper(hyper, gscale=self.grad_scale, **self._advance(group))
+        return hyper
 
     @torch.no_grad()
-    def step_range(self, owner, lo: int, hi: int, hp: dict) -> None:
+    def step_range(self, owner, lo: int, hi: int, hyper: torch.Tensor) -> None:
         """Schedule-Free AdamW on flat elements [lo, hi) of `owner` (multiples of 4), on the current stream."""
         from ..ops import kernels as K
-        K.sfadamw_step(owner.data[lo:hi], owner.sf_z[lo:hi], owner.sf_v[lo:hi], owner.grad[lo:hi], owner.w16[lo:hi],
-                       gscale=self.grad_scale, zero_grad=True, **hp)
+        K.sfadamw_dyn_step(owner.data[lo:hi], owner.sf_z[lo:hi], owner.sf_v[lo:hi], owner.grad[lo:hi], owner.w16[lo:hi],
+                           hyper)
 
     def end_ranged_step(self, owner) -> None:
         self.param_groups[0]["k"] += 1
