@@ -9,12 +9,14 @@
 // linear space is at least as accurate as the reference's fp32 log-space path.
 //
 // Layout: k, u, h are bf16 [B, T, C] with a row stride (k and u are usually the
-// two column halves of one GEMM output).  One CTA owns 64 channels of one batch
-// row and walks T in order, so no inter-CTA communication is needed.  Raw tiles
-// arrive through a 3-stage TMA ring.  Inside a super-step the four warps each
-// take a slice of consecutive time steps, scan it locally from a zero state
-// (keeping per-step (prefix-product, local value) pairs in registers), exchange
-// slice aggregates through shared memory, and finish with one FMA per element.
+// two column halves of one GEMM output).  A cluster of S CTAs (S = 1: one CTA)
+// owns 64 channels of one batch row and walks T in rounds of S super-steps, one
+// per CTA.  Raw tiles arrive through a 3-stage TMA ring.  Inside a super-step the
+// four warps each take a slice of consecutive time steps, scan it locally from a
+// zero state (keeping per-step (prefix-product, local value) pairs in registers),
+// exchange slice aggregates - through shared memory in one CTA, with st.async
+// into every CTA's table (counted on a barrier there) in a cluster - and finish
+// with one FMA per element.
 // Results go to a per-warp staging tile and leave with one bulk tensor store
 // per slice (which also clips the ragged ends of T and C); super-steps that lie
 // wholly inside T run a variant of the slice loop without any bounds handling.
@@ -29,33 +31,18 @@
 namespace grb {
 
 constexpr int SC_CH = 64;
-#ifndef GRB_SCAN_WARPS
-#define GRB_SCAN_WARPS 4
-#endif
-#ifndef GRB_SCAN_FSTEPS
-#define GRB_SCAN_FSTEPS 16
-#endif
-#ifndef GRB_SCAN_RSTEPS
-#define GRB_SCAN_RSTEPS 8
-#endif
-constexpr int SC_NW = GRB_SCAN_WARPS;               // warps per CTA: each takes a slice of a super-step
-constexpr int SC_THREADS = 32 * SC_NW;
-#ifndef GRB_SCAN_STAGES
-#define GRB_SCAN_STAGES 3
-#endif
-constexpr int SC_STAGES = GRB_SCAN_STAGES;
-
-constexpr int F_STEPS = GRB_SCAN_FSTEPS;                       // steps per warp per super-step
-constexpr int F_TS = SC_NW * F_STEPS;
-constexpr int F_TILE = F_TS * SC_CH * 2;          // bytes of one tensor tile
-constexpr int F_STAGE_BYTES = 2 * F_TILE;         // k, u
-constexpr int F_OUT_WARP = F_STEPS * SC_CH * 2;   // staging tile of one warp: its slice of h
-
-constexpr int R_STEPS = GRB_SCAN_RSTEPS;
-constexpr int R_TS = SC_NW * R_STEPS;
-constexpr int R_TILE = R_TS * SC_CH * 2;
-constexpr int R_STAGE_BYTES = 4 * R_TILE;         // k, u, h_prev, g
-constexpr int R_OUT_WARP = 2 * R_STEPS * SC_CH * 2;   // staging tiles of one warp: its slices of dk and du
+// Sizes of a kernel of NW warps that each take STEPS time steps of a super-step; NIN tensors in, NOUT tensors out,
+// input ring of STAGES super-steps.
+template <int NW_, int STEPS_, int STAGES_, int NIN, int NOUT>
+struct ScanShape {
+  static constexpr int NW = NW_, STEPS = STEPS_, STAGES = STAGES_;
+  static constexpr int THREADS = 32 * NW;
+  static constexpr int TS = NW * STEPS;                 // time steps of a super-step
+  static constexpr int TILE = TS * SC_CH * 2;           // bytes of one tensor tile
+  static constexpr int STAGE = NIN * TILE;
+  static constexpr int OUT_WARP = NOUT * STEPS * SC_CH * 2;   // staging tiles of one warp
+  static constexpr int smem(int S) { return 128 + STAGES * STAGE + NW * OUT_WARP + 1024 * (NW + (S > 1 ? S : 0)) + 64; }
+};
 
 __device__ __forceinline__ float ex2f(float x) {
   float y;
@@ -134,6 +121,95 @@ __device__ __forceinline__ void tma_store_3d(const void* desc, const void* smem_
 // The staging tile a bulk store was issued from may be rewritten / released once the store has read it.
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes into CTA `cta`'s copy of a shared-memory location, counted on that CTA's copy of `bar`.
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t bar, uint32_t cta, float4 v) {
+  asm volatile(
+      "{\n"
+      ".reg .b32 ra, rb;\n"
+      "mapa.shared::cluster.u32 ra, %0, %2;\n"
+      "mapa.shared::cluster.u32 rb, %1, %2;\n"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [ra], {%3, %4, %5, %6}, [rb];\n"
+      "}\n" ::"r"(addr), "r"(bar), "r"(cta), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+      : "memory");
+}
+
+// What both kernels keep beside the input ring: barriers, and aggregates (prefix product and value, two channels per lane)
+// for two rounds: of the CTA's warps, and of the cluster's CTAs.
+template <int NW>
+struct Exchange {
+  uint64_t* full;      // [STAGES] input tiles have landed
+  uint64_t* got;       // [2] the aggregates of all CTAs have landed
+  float4* loc;         // [2][NW][32]
+  float4* all;         // [2][S][32]
+  int S, rank;
+
+  __device__ __forceinline__ float4* warp_slot(int par, int w) const { return loc + (par * NW + w) * 32; }
+  __device__ __forceinline__ float4* cta_slot(int par, int r) const { return all + (par * S + r) * 32; }
+  __device__ __forceinline__ void arm(int par) const { mbar_expect_tx(&got[par], S * 512); }
+
+  // a then b, in the direction of the recurrence
+  static __device__ __forceinline__ float4 chain(float4 a, float4 b) {
+    return make_float4(a.x * b.x, fmaf(b.x, a.y, b.y), a.z * b.z, fmaf(b.z, a.w, b.w));
+  }
+  static __device__ __forceinline__ void apply(float4 x, float& c0, float& c1) {
+    c0 = fmaf(x.x, c0, x.y);
+    c1 = fmaf(x.z, c1, x.w);
+  }
+
+  // Publish this warp's aggregate, wait for the others', advance the carried state (c0, c1) over the whole round and return
+  // in (in0, in1) the state that enters this warp's slice.  REV: time runs backwards.  False (in every thread of the CTA)
+  // when an earlier wait ran out in some thread (ok); its own wait clears ok, for the next round.  A table is written again two rounds later, by warps that have then passed the round between, which
+  // every reader of this table enters only after its reads.
+  template <bool CL, bool REV>
+  __device__ __forceinline__ bool trade(int round, int warp, int lane, float4 mine, bool& ok, float& c0, float& c1,
+                                        float& in0, float& in1) const {
+    const int par = round & 1;
+    warp_slot(par, warp)[lane] = mine;
+    if (!__syncthreads_and(ok ? 1 : 0)) return false;
+    if constexpr (CL) {
+      if (warp < S) {                       // NW >= S: warp d sends the CTA's aggregate to CTA d
+        float4 tot = warp_slot(par, REV ? NW - 1 : 0)[lane];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) tot = chain(tot, warp_slot(par, REV ? NW - 1 - w : w)[lane]);
+        st_async(smem_u32(cta_slot(par, rank) + lane), smem_u32(&got[par]), warp, tot);
+      }
+      if (!__all_sync(0xffffffffu, mbar_wait(&got[par], (round >> 1) & 1))) ok = false;
+      if (threadIdx.x == 0) arm(par);
+      for (int i = 0; i < S; ++i) {
+        const int r = REV ? S - 1 - i : i;
+        if (r == rank) { in0 = c0; in1 = c1; }
+        apply(cta_slot(par, r)[lane], c0, c1);
+      }
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        const int w = REV ? NW - 1 - i : i;
+        if (REV ? w > warp : w < warp) apply(warp_slot(par, w)[lane], in0, in1);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        const int w = REV ? NW - 1 - i : i;
+        if (w == warp) { in0 = c0; in1 = c1; }
+        apply(warp_slot(par, w)[lane], c0, c1);
+      }
+    }
+    return true;
+  }
+};
+
 struct ScanFwdArgs {
   int B, T, C;
   const float* h0;       // [B, C] or null
@@ -145,35 +221,51 @@ struct ScanFwdArgs {
 
 // TMA_OUT: h leaves through the staging tile and a bulk tensor store (needs a tensor map of h: 16-byte aligned base
 // and row stride); otherwise every lane stores its own values.
-template <bool TMA_OUT>
-__global__ void __launch_bounds__(SC_THREADS)
+// CL: launched as clusters of S CTAs along T (x = channel group * S + rank).
+template <typename Sh, bool TMA_OUT, bool CL>
+__global__ void __launch_bounds__(Sh::THREADS)
 scan_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
                 const __grid_constant__ CUtensorMap tmH, const ScanFwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  uint8_t* out_stage = smem + SC_STAGES * F_STAGE_BYTES;                      // [SC_NW][F_STEPS][64] bf16
-  uint64_t* full = reinterpret_cast<uint64_t*>(out_stage + SC_NW * F_OUT_WARP);
-  float2* agg = reinterpret_cast<float2*>(full + SC_STAGES);   // [2][SC_NW][64]
+  constexpr int STEPS = Sh::STEPS;
+  uint8_t* out_stage = smem + Sh::STAGES * Sh::STAGE;                          // [NW][STEPS][64] bf16
+  Exchange<Sh::NW> ex;
+  ex.S = CL ? static_cast<int>(cluster_size()) : 1;
+  ex.rank = CL ? static_cast<int>(cluster_rank()) : 0;
+  ex.loc = reinterpret_cast<float4*>(out_stage + Sh::NW * Sh::OUT_WARP);
+  ex.all = ex.loc + 2 * Sh::NW * 32;
+  ex.full = reinterpret_cast<uint64_t*>(ex.all + (CL ? 2 * ex.S * 32 : 0));
+  ex.got = ex.full + Sh::STAGES;
+  uint64_t* full = ex.full;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.y, c0 = blockIdx.x * SC_CH;
+  const int b = blockIdx.y, c0 = (blockIdx.x / ex.S) * SC_CH;
   const int ch = c0 + 2 * lane;
-  const int nss = (p.T + F_TS - 1) / F_TS;
+  const int nss = (p.T + Sh::TS - 1) / Sh::TS;
+  const int rounds = (nss + ex.S - 1) / ex.S;
+
+  auto issue = [&](int r) {                     // thread 0: this CTA's super-step of round r (all zeros beyond T)
+    const int stage = r % Sh::STAGES, t0 = (r * ex.S + ex.rank) * Sh::TS;
+    mbar_expect_tx(&full[stage], Sh::STAGE);
+    tma_load_3d(smem + stage * Sh::STAGE, &tmK, &full[stage], c0, t0, b);
+    tma_load_3d(smem + stage * Sh::STAGE + Sh::TILE, &tmU, &full[stage], c0, t0, b);
+  };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < SC_STAGES; ++s) mbar_init(&full[s], 1);
+    for (int s = 0; s < Sh::STAGES; ++s) mbar_init(&full[s], 1);
+    mbar_init(&ex.got[0], 1);
+    mbar_init(&ex.got[1], 1);
     fence_mbar_init();
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmU);
     if (TMA_OUT) tma_prefetch_desc(&tmH);
   }
-  __syncthreads();
+  if constexpr (CL) cluster_sync();             // every CTA's barriers are ready for the others' aggregates
+  else __syncthreads();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < SC_STAGES && s < nss; ++s) {
-      mbar_expect_tx(&full[s], F_STAGE_BYTES);
-      tma_load_3d(smem + s * F_STAGE_BYTES, &tmK, &full[s], c0, s * F_TS, b);
-      tma_load_3d(smem + s * F_STAGE_BYTES + F_TILE, &tmU, &full[s], c0, s * F_TS, b);
-    }
+    if (CL) { ex.arm(0); ex.arm(1); }
+    for (int r = 0; r < Sh::STAGES && r < rounds; ++r) issue(r);
   }
 
   float c_0 = 0.f, c_1 = 0.f;   // carried hidden state of this lane's two channels
@@ -181,24 +273,27 @@ scan_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (ch < p.C) c_0 = p.h0[static_cast<size_t>(b) * p.C + ch];
     if (ch + 1 < p.C) c_1 = p.h0[static_cast<size_t>(b) * p.C + ch + 1];
   }
-  uint32_t* my_stage = reinterpret_cast<uint32_t*>(out_stage + warp * F_OUT_WARP) + lane;
+  uint32_t* my_stage = reinterpret_cast<uint32_t*>(out_stage + warp * Sh::OUT_WARP) + lane;
 
-  for (int ss = 0; ss < nss; ++ss) {
-    const int stage = ss % SC_STAGES;
-    const uint32_t phase = (ss / SC_STAGES) & 1;
-    const int par = ss & 1;
-    bool ok = mbar_wait(&full[stage], phase);
+  int done = 0;
+  bool ok = true;
+  for (int r = 0; r < rounds; ++r) {
+    const int stage = r % Sh::STAGES;
+    const uint32_t phase = (r / Sh::STAGES) & 1;
+    const int ss = r * ex.S + ex.rank;
+    if (!mbar_wait(&full[stage], phase)) ok = false;
 
-    float2 S[F_STEPS], P[F_STEPS];
-    const int tbase = ss * F_TS + warp * F_STEPS;
+    float2 S[STEPS], P[STEPS];
+    const int tbase = ss * Sh::TS + warp * STEPS;
+    float4 mine;
     {
-      const uint32_t* sk = reinterpret_cast<const uint32_t*>(smem + stage * F_STAGE_BYTES) + (warp * F_STEPS) * (SC_CH / 2) + lane;
-      const uint32_t* su = sk + F_TILE / 4;
+      const uint32_t* sk = reinterpret_cast<const uint32_t*>(smem + stage * Sh::STAGE) + (warp * STEPS) * (SC_CH / 2) + lane;
+      const uint32_t* su = sk + Sh::TILE / 4;
       float2 sc = splat2(0.f), q = splat2(1.f);
       // local scan of the slice from a zero state; `masked` adds the handling of time steps at or beyond T
       auto slice = [&](auto masked) {
 #pragma unroll
-        for (int i = 0; i < F_STEPS; ++i) {
+        for (int i = 0; i < STEPS; ++i) {
           const uint32_t kk = clamp_below_bf16x2(sk[i * (SC_CH / 2)]), uu = clamp_below_bf16x2(su[i * (SC_CH / 2)]);
           float2 a, bb;
           gate_act_fwd2(kk, uu, a, bb);
@@ -208,38 +303,20 @@ scan_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
           S[i] = sc; P[i] = q;
         }
       };
-      if ((ss + 1) * F_TS <= p.T) slice(std::false_type{});
+      if ((ss + 1) * Sh::TS <= p.T) slice(std::false_type{});
       else slice(std::true_type{});
-      agg[(par * SC_NW + warp) * SC_CH + 2 * lane] = make_float2(q.x, sc.x);
-      agg[(par * SC_NW + warp) * SC_CH + 2 * lane + 1] = make_float2(q.y, sc.y);
+      mine = make_float4(q.x, sc.x, q.y, sc.y);
     }
-    const int all_ok = __syncthreads_and(ok ? 1 : 0);
-    if (!all_ok) {
-      if (threadIdx.x == 0) atomicExch(p.err, 11);
-      break;
-    }
-    if (threadIdx.x == 0 && ss + SC_STAGES < nss) {
-      const int nx = ss + SC_STAGES;
-      mbar_expect_tx(&full[stage], F_STAGE_BYTES);
-      tma_load_3d(smem + stage * F_STAGE_BYTES, &tmK, &full[stage], c0, nx * F_TS, b);
-      tma_load_3d(smem + stage * F_STAGE_BYTES + F_TILE, &tmU, &full[stage], c0, nx * F_TS, b);
-    }
-    // state entering this warp's slice, and the state leaving the super-step
-    float in0 = c_0, in1 = c_1;
-#pragma unroll
-    for (int w = 0; w < SC_NW; ++w) {
-      const float2 x0 = agg[(par * SC_NW + w) * SC_CH + 2 * lane];
-      const float2 x1 = agg[(par * SC_NW + w) * SC_CH + 2 * lane + 1];
-      c_0 = fmaf(x0.x, c_0, x0.y);
-      c_1 = fmaf(x1.x, c_1, x1.y);
-      if (w + 1 == warp) { in0 = c_0; in1 = c_1; }
-    }
+    float in0, in1;                             // state entering this warp's slice
+    if (!ex.template trade<CL, false>(r, warp, lane, mine, ok, c_0, c_1, in0, in1)) break;
+    done = r + 1;
+    if (threadIdx.x == 0 && r + Sh::STAGES < rounds) issue(r + Sh::STAGES);   // every warp of the CTA has read the stage
     if constexpr (TMA_OUT) {
       if (tbase < p.T) {                        // uniform across the warp
         if (lane == 0) tma_store_wait_read();   // the store issued a super-step ago has read the tile
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < F_STEPS; ++i)
+        for (int i = 0; i < STEPS; ++i)
         {
           const float2 v = ffma2(P[i], make_float2(in0, in1), S[i]);
           my_stage[i * (SC_CH / 2)] = pack_bf16(v.x, v.y);
@@ -247,12 +324,12 @@ scan_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         fence_proxy_async_smem();
         __syncwarp();
         // rows at or beyond T and channels at or beyond C are clipped by the store
-        if (lane == 0) tma_store_3d(&tmH, out_stage + warp * F_OUT_WARP, c0, tbase, b);
+        if (lane == 0) tma_store_3d(&tmH, out_stage + warp * Sh::OUT_WARP, c0, tbase, b);
       }
     } else if (ch < p.C) {
       __nv_bfloat16* hp = p.h + (static_cast<size_t>(b) * p.T + tbase) * p.ldh + ch;
 #pragma unroll
-      for (int i = 0; i < F_STEPS; ++i) {
+      for (int i = 0; i < STEPS; ++i) {
         if (tbase + i < p.T) {
           const float v0 = fmaf(P[i].x, in0, S[i].x);
           const float v1 = fmaf(P[i].y, in1, S[i].y);
@@ -263,7 +340,11 @@ scan_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     }
   }
   if (TMA_OUT && lane == 0) tma_store_wait_read();   // before the shared memory is released
-  if (warp == 0 && p.h_last) {
+  if (!ok) atomicExch(p.err, 11);
+  if (done < rounds && threadIdx.x == 0)             // a wait ran out: what was issued may still be landing
+    for (int r = done; r < rounds && r < done + Sh::STAGES; ++r) mbar_wait(&full[r % Sh::STAGES], (r / Sh::STAGES) & 1);
+  if constexpr (CL) cluster_sync();                  // nobody's aggregates land in a CTA that has gone
+  if (ex.rank == 0 && warp == 0 && p.h_last) {
     if (ch < p.C) p.h_last[static_cast<size_t>(b) * p.C + ch] = c_0;
     if (ch + 1 < p.C) p.h_last[static_cast<size_t>(b) * p.C + ch + 1] = c_1;
   }
@@ -285,42 +366,56 @@ struct ScanBwdArgs {
 //   mu_t = a_t * (G_t + mu_{t+1})      (gradient reaching h_{t-1} through step t)
 //   lambda_t = G_t + mu_{t+1}          (total gradient of h_t)
 //   dk_t = lambda_t * (g(u_t) - h_{t-1}) * z_t * a_t,   du_t = lambda_t * z_t * g'(u_t)
-// TMA_OUT as in the forward kernel (tensor maps of dk and du).
-template <bool TMA_OUT>
-__global__ void __launch_bounds__(SC_THREADS)
+// TMA_OUT (tensor maps of dk and du) and CL as in the forward kernel; the rounds run from the end of T, the time order of
+// the CTAs inside a round is the same.
+template <typename Sh, bool TMA_OUT, bool CL>
+__global__ void __launch_bounds__(Sh::THREADS)
 scan_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
                 const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmG,
                 const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDU, const ScanBwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  uint8_t* out_stage = smem + SC_STAGES * R_STAGE_BYTES;                      // [SC_NW][dk, du][R_STEPS][64] bf16
-  uint64_t* full = reinterpret_cast<uint64_t*>(out_stage + SC_NW * R_OUT_WARP);
-  float2* agg = reinterpret_cast<float2*>(full + SC_STAGES);   // [2][SC_NW][64]
+  constexpr int STEPS = Sh::STEPS;
+  uint8_t* out_stage = smem + Sh::STAGES * Sh::STAGE;                          // [NW][dk, du][STEPS][64] bf16
+  Exchange<Sh::NW> ex;
+  ex.S = CL ? static_cast<int>(cluster_size()) : 1;
+  ex.rank = CL ? static_cast<int>(cluster_rank()) : 0;
+  ex.loc = reinterpret_cast<float4*>(out_stage + Sh::NW * Sh::OUT_WARP);
+  ex.all = ex.loc + 2 * Sh::NW * 32;
+  ex.full = reinterpret_cast<uint64_t*>(ex.all + (CL ? 2 * ex.S * 32 : 0));
+  ex.got = ex.full + Sh::STAGES;
+  uint64_t* full = ex.full;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.y, c0 = blockIdx.x * SC_CH;
+  const int b = blockIdx.y, c0 = (blockIdx.x / ex.S) * SC_CH;
   const int ch = c0 + 2 * lane;
-  const int nss = (p.T + R_TS - 1) / R_TS;
+  const int nss = (p.T + Sh::TS - 1) / Sh::TS;
+  const int rounds = (nss + ex.S - 1) / ex.S;
 
-  auto issue = [&](int j, int stage) {
-    const int t0 = (nss - 1 - j) * R_TS;
-    uint8_t* s = smem + stage * R_STAGE_BYTES;
-    mbar_expect_tx(&full[stage], R_STAGE_BYTES);
+  auto issue = [&](int r) {
+    const int stage = r % Sh::STAGES, t0 = ((rounds - 1 - r) * ex.S + ex.rank) * Sh::TS;
+    uint8_t* s = smem + stage * Sh::STAGE;
+    mbar_expect_tx(&full[stage], Sh::STAGE);
     tma_load_3d(s, &tmK, &full[stage], c0, t0, b);
-    tma_load_3d(s + R_TILE, &tmU, &full[stage], c0, t0, b);
-    tma_load_3d(s + 2 * R_TILE, &tmH, &full[stage], c0, t0 - 1, b);   // h_{t-1}; row -1 reads zeros
-    tma_load_3d(s + 3 * R_TILE, &tmG, &full[stage], c0, t0, b);
+    tma_load_3d(s + Sh::TILE, &tmU, &full[stage], c0, t0, b);
+    tma_load_3d(s + 2 * Sh::TILE, &tmH, &full[stage], c0, t0 - 1, b);   // h_{t-1}; row -1 reads zeros
+    tma_load_3d(s + 3 * Sh::TILE, &tmG, &full[stage], c0, t0, b);
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < SC_STAGES; ++s) mbar_init(&full[s], 1);
+    for (int s = 0; s < Sh::STAGES; ++s) mbar_init(&full[s], 1);
+    mbar_init(&ex.got[0], 1);
+    mbar_init(&ex.got[1], 1);
     fence_mbar_init();
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmU); tma_prefetch_desc(&tmH); tma_prefetch_desc(&tmG);
     if (TMA_OUT) { tma_prefetch_desc(&tmDK); tma_prefetch_desc(&tmDU); }
   }
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int s = 0; s < SC_STAGES && s < nss; ++s) issue(s, s);
+  if constexpr (CL) cluster_sync();             // every CTA's barriers are ready for the others' aggregates
+  else __syncthreads();
+  if (threadIdx.x == 0) {
+    if (CL) { ex.arm(0); ex.arm(1); }
+    for (int r = 0; r < Sh::STAGES && r < rounds; ++r) issue(r);
+  }
 
   float h00 = 0.f, h01 = 0.f;
   if (p.h0) {
@@ -332,35 +427,37 @@ scan_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (ch < p.C) m_0 = p.dh_last[static_cast<size_t>(b) * p.C + ch];
     if (ch + 1 < p.C) m_1 = p.dh_last[static_cast<size_t>(b) * p.C + ch + 1];
   }
-  uint32_t* my_dk = reinterpret_cast<uint32_t*>(out_stage + warp * R_OUT_WARP) + lane;
-  uint32_t* my_du = my_dk + R_OUT_WARP / 8;
+  uint32_t* my_dk = reinterpret_cast<uint32_t*>(out_stage + warp * Sh::OUT_WARP) + lane;
+  uint32_t* my_du = my_dk + Sh::OUT_WARP / 8;
 
-  for (int j = 0; j < nss; ++j) {
-    const int ss = nss - 1 - j;
-    const int stage = j % SC_STAGES;
-    const uint32_t phase = (j / SC_STAGES) & 1;
-    const int par = j & 1;
-    const int tbase = ss * R_TS + warp * R_STEPS;
-    const bool inside = ss > 0 && (ss + 1) * R_TS <= p.T;     // no step of this super-step is 0 or >= T
+  int done = 0;
+  bool ok = true;
+  for (int r = 0; r < rounds; ++r) {
+    const int ss = (rounds - 1 - r) * ex.S + ex.rank;
+    const int stage = r % Sh::STAGES;
+    const uint32_t phase = (r / Sh::STAGES) & 1;
+    const int tbase = ss * Sh::TS + warp * STEPS;
+    const bool inside = ss > 0 && (ss + 1) * Sh::TS <= p.T;     // no step of this super-step is 0 or >= T
     // row scales of this warp's steps, requested before the wait on the tiles so that their latency is hidden
-    float rsc[R_STEPS];
+    float rsc[STEPS];
 #pragma unroll
-    for (int i = 0; i < R_STEPS; ++i)
+    for (int i = 0; i < STEPS; ++i)
       rsc[i] = (p.rowscale && (inside || tbase + i < p.T)) ? __ldg(p.rowscale + static_cast<size_t>(b) * p.T + tbase + i) : 1.f;
-    bool ok = mbar_wait(&full[stage], phase);
+    if (!mbar_wait(&full[stage], phase)) ok = false;
 
     // per step: lambda_loc = G + mu_loc(next), rn = prod of a over later steps of the slice, c1, c2
-    float2 L[R_STEPS], Q[R_STEPS], C1[R_STEPS], C2[R_STEPS];
+    float2 L[STEPS], Q[STEPS], C1[STEPS], C2[STEPS];
+    float4 mine;
     {
-      const uint32_t* sk = reinterpret_cast<const uint32_t*>(smem + stage * R_STAGE_BYTES) + (warp * R_STEPS) * (SC_CH / 2) + lane;
-      const uint32_t* su = sk + R_TILE / 4;
-      const uint32_t* sh = sk + 2 * (R_TILE / 4);
-      const uint32_t* sg = sk + 3 * (R_TILE / 4);
+      const uint32_t* sk = reinterpret_cast<const uint32_t*>(smem + stage * Sh::STAGE) + (warp * STEPS) * (SC_CH / 2) + lane;
+      const uint32_t* su = sk + Sh::TILE / 4;
+      const uint32_t* sh = sk + 2 * (Sh::TILE / 4);
+      const uint32_t* sg = sk + 3 * (Sh::TILE / 4);
       float2 mu = splat2(0.f), rr = splat2(1.f);
       auto slice = [&](auto masked) {
         constexpr bool MASKED = decltype(masked)::value;
 #pragma unroll
-        for (int i = R_STEPS - 1; i >= 0; --i) {
+        for (int i = STEPS - 1; i >= 0; --i) {
           const uint32_t kk = clamp_below_bf16x2(sk[i * (SC_CH / 2)]), uu = clamp_below_bf16x2(su[i * (SC_CH / 2)]);
           const uint32_t hh = sh[i * (SC_CH / 2)], gg = sg[i * (SC_CH / 2)];
           float2 a, z, g, d;
@@ -381,31 +478,18 @@ scan_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       };
       if (inside) slice(std::false_type{});
       else slice(std::true_type{});
-      agg[(par * SC_NW + warp) * SC_CH + 2 * lane] = make_float2(rr.x, mu.x);
-      agg[(par * SC_NW + warp) * SC_CH + 2 * lane + 1] = make_float2(rr.y, mu.y);
+      mine = make_float4(rr.x, mu.x, rr.y, mu.y);
     }
-    const int all_ok = __syncthreads_and(ok ? 1 : 0);
-    if (!all_ok) {
-      if (threadIdx.x == 0) atomicExch(p.err, 12);
-      break;
-    }
-    if (threadIdx.x == 0 && j + SC_STAGES < nss) issue(j + SC_STAGES, stage);
-
-    float in0 = m_0, in1 = m_1;
-#pragma unroll
-    for (int w = SC_NW - 1; w >= 0; --w) {
-      if (w == warp) { in0 = m_0; in1 = m_1; }
-      const float2 x0 = agg[(par * SC_NW + w) * SC_CH + 2 * lane];
-      const float2 x1 = agg[(par * SC_NW + w) * SC_CH + 2 * lane + 1];
-      m_0 = fmaf(x0.x, m_0, x0.y);
-      m_1 = fmaf(x1.x, m_1, x1.y);
-    }
+    float in0, in1;
+    if (!ex.template trade<CL, true>(r, warp, lane, mine, ok, m_0, m_1, in0, in1)) break;
+    done = r + 1;
+    if (threadIdx.x == 0 && r + Sh::STAGES < rounds) issue(r + Sh::STAGES);
     if constexpr (TMA_OUT) {
       if (tbase < p.T) {                        // uniform across the warp
         if (lane == 0) tma_store_wait_read();   // the stores issued a super-step ago have read the tiles
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < R_STEPS; ++i) {
+        for (int i = 0; i < STEPS; ++i) {
           const float2 l = fmul2(ffma2(Q[i], make_float2(in0, in1), L[i]), splat2(rsc[i]));
           const float2 vk = fmul2(l, C1[i]), vu = fmul2(l, C2[i]);
           my_dk[i * (SC_CH / 2)] = pack_bf16(vk.x, vk.y);
@@ -414,14 +498,14 @@ scan_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {                        // rows at or beyond T and channels at or beyond C are clipped
-          tma_store_3d(&tmDK, out_stage + warp * R_OUT_WARP, c0, tbase, b);
-          tma_store_3d(&tmDU, out_stage + warp * R_OUT_WARP + R_OUT_WARP / 2, c0, tbase, b);
+          tma_store_3d(&tmDK, out_stage + warp * Sh::OUT_WARP, c0, tbase, b);
+          tma_store_3d(&tmDU, out_stage + warp * Sh::OUT_WARP + Sh::OUT_WARP / 2, c0, tbase, b);
         }
       }
     } else if (ch < p.C) {
       const size_t row0 = (static_cast<size_t>(b) * p.T + tbase) * p.ldd + ch;
 #pragma unroll
-      for (int i = 0; i < R_STEPS; ++i) {
+      for (int i = 0; i < STEPS; ++i) {
         if (tbase + i < p.T) {
           const float l0 = fmaf(Q[i].x, in0, L[i].x) * rsc[i];
           const float l1 = fmaf(Q[i].y, in1, L[i].y) * rsc[i];
@@ -438,23 +522,119 @@ scan_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     }
   }
   if (TMA_OUT && lane == 0) tma_store_wait_read();   // before the shared memory is released
-  if (warp == 0 && p.dh0) {
+  if (!ok) atomicExch(p.err, 12);
+  if (done < rounds && threadIdx.x == 0)             // a wait ran out: what was issued may still be landing
+    for (int r = done; r < rounds && r < done + Sh::STAGES; ++r) mbar_wait(&full[r % Sh::STAGES], (r / Sh::STAGES) & 1);
+  if constexpr (CL) cluster_sync();                  // nobody's aggregates land in a CTA that has gone
+  if (ex.rank == 0 && warp == 0 && p.dh0) {
     if (ch < p.C) p.dh0[static_cast<size_t>(b) * p.C + ch] = m_0;
     if (ch + 1 < p.C) p.dh0[static_cast<size_t>(b) * p.C + ch + 1] = m_1;
   }
 }
 
-constexpr int F_SMEM = SC_STAGES * F_STAGE_BYTES + SC_NW * F_OUT_WARP + 128 + SC_STAGES * 8 + 2 * SC_NW * SC_CH * 8;
-constexpr int R_SMEM = SC_STAGES * R_STAGE_BYTES + SC_NW * R_OUT_WARP + 128 + SC_STAGES * 8 + 2 * SC_NW * SC_CH * 8;
+template <int NW, int STEPS, int STAGES> using FwdShape = ScanShape<NW, STEPS, STAGES, 2, 1>;   // k, u -> h
+template <int NW, int STEPS, int STAGES> using BwdShape = ScanShape<NW, STEPS, STAGES, 4, 2>;   // k, u, h_prev, g -> dk, du
+// One CTA per channel group: four warps with long slices, three CTAs per SM.  Clusters serve launches of few channel groups,
+// which are bound by the latency of a round (a slice, two barriers, the trip to the other CTAs: about 3 us), so their CTAs
+// have eight warps.  B1 x T2047 x C3072 (48 channel groups): forward 42.6 us on one CTA each, 14.7 us on eight; backward 71.7
+// and 25.4 us; B3 x T999 x C3072: 22.8 -> 14.9 and 37.7 -> 26.2 us.
+using Fwd1 = FwdShape<4, 16, 3>;
+using FwdC = FwdShape<8, 16, 2>;        // sequences of several rounds: half as many rounds as with 8 steps
+using FwdCShort = FwdShape<8, 8, 2>;    // short ones: more CTAs have a super-step
+using Bwd1 = BwdShape<4, 8, 3>;
+using BwdC = BwdShape<8, 8, 2>;
 // All (C / 64) x B CTAs of the 1B and 3B shapes are meant to be resident at once: three per SM.
-static_assert(3 * (F_SMEM + 1024) <= 233472 && 3 * (R_SMEM + 1024) <= 233472, "three scan CTAs per SM must fit");
+static_assert(3 * (Fwd1::smem(1) + 1024) <= 233472 && 3 * (Bwd1::smem(1) + 1024) <= 233472, "three scan CTAs per SM must fit");
 
-template <typename Kern>
-static int allow_smem(Kern kern, int bytes, bool& done) {
-  if (done) return 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return -4;
-  done = true;
-  return 0;
+// CTAs per cluster: T is split as long as all clusters fit on the machine at once and each CTA has a super-step of its own.
+template <typename Sh, typename Kern>
+static int pick_split(Kern kern, int groups, int T) {
+  static int fit[4] = {-1, -1, -1, -1};      // clusters of 2, 4, 8 CTAs that are resident together
+  const int nss = (T + Sh::TS - 1) / Sh::TS;
+  int S = 1;
+  for (int i = 1; i < 4; ++i) {
+    const int n = 1 << i;
+    if (n > nss) break;
+    if (fit[i] < 0) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::smem(8));
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(n);
+      cfg.blockDim = dim3(Sh::THREADS);
+      cfg.dynamicSmemBytes = Sh::smem(n);
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int q = 0;
+      fit[i] = cudaOccupancyMaxActiveClusters(&q, kern, &cfg) == cudaSuccess ? q : 0;
+    }
+    if (groups > fit[i]) break;
+    S = n;
+  }
+  return S;
+}
+
+template <typename Sh, typename Kern, typename... Args>
+static int launch_scan(Kern kern, size_t& granted, int groups, int B, int S, void* st, const Args&... args) {
+  const int smem = Sh::smem(S);
+  if (static_cast<size_t>(smem) > granted) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
+    granted = smem;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(groups * S, B);
+  cfg.blockDim = dim3(Sh::THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = reinterpret_cast<cudaStream_t>(st);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? 0 : -5;
+}
+
+struct ScanIo {                       // inputs of both directions (h and g are the backward's)
+  const void *k, *u; int64_t ldku;
+  const void* h; int64_t ldh;
+  const void* g; int64_t ldg;
+};
+
+template <typename Sh, bool CL>
+static int run_fwd(const ScanIo& io, const ScanFwdArgs& a, int S, void* st) {
+  CUtensorMap tmK, tmU, tmH;
+  int rc = make_tmap_btc_bf16(&tmK, io.k, a.C, a.T, a.B, io.ldku, SC_CH, Sh::TS);
+  if (rc) return rc;
+  rc = make_tmap_btc_bf16(&tmU, io.u, a.C, a.T, a.B, io.ldku, SC_CH, Sh::TS);
+  if (rc) return rc;
+  // the output leaves through bulk tensor stores when its layout allows a tensor map (16-byte aligned base and rows)
+  const bool tma_out = make_tmap_btc_bf16(&tmH, a.h, a.C, a.T, a.B, a.ldh, SC_CH, Sh::STEPS) == 0;
+  if (!tma_out) tmH = tmK;
+  static size_t granted[2] = {};
+  const int groups = (a.C + SC_CH - 1) / SC_CH;
+  return tma_out ? launch_scan<Sh>(scan_fwd_kernel<Sh, true, CL>, granted[1], groups, a.B, S, st, tmK, tmU, tmH, a)
+                 : launch_scan<Sh>(scan_fwd_kernel<Sh, false, CL>, granted[0], groups, a.B, S, st, tmK, tmU, tmH, a);
+}
+
+template <typename Sh, bool CL>
+static int run_bwd(const ScanIo& io, const ScanBwdArgs& a, int S, void* st) {
+  CUtensorMap tmK, tmU, tmH, tmG, tmDK, tmDU;
+  int rc = make_tmap_btc_bf16(&tmK, io.k, a.C, a.T, a.B, io.ldku, SC_CH, Sh::TS);
+  if (rc) return rc;
+  rc = make_tmap_btc_bf16(&tmU, io.u, a.C, a.T, a.B, io.ldku, SC_CH, Sh::TS);
+  if (rc) return rc;
+  rc = make_tmap_btc_bf16(&tmH, io.h, a.C, a.T, a.B, io.ldh, SC_CH, Sh::TS);
+  if (rc) return rc;
+  rc = make_tmap_btc_bf16(&tmG, io.g, a.C, a.T, a.B, io.ldg, SC_CH, Sh::TS);
+  if (rc) return rc;
+  const bool tma_out = make_tmap_btc_bf16(&tmDK, a.dk, a.C, a.T, a.B, a.ldd, SC_CH, Sh::STEPS) == 0 &&
+                       make_tmap_btc_bf16(&tmDU, a.du, a.C, a.T, a.B, a.ldd, SC_CH, Sh::STEPS) == 0;
+  if (!tma_out) tmDK = tmDU = tmK;
+  static size_t granted[2] = {};
+  const int groups = (a.C + SC_CH - 1) / SC_CH;
+  return tma_out ? launch_scan<Sh>(scan_bwd_kernel<Sh, true, CL>, granted[1], groups, a.B, S, st, tmK, tmU, tmH, tmG, tmDK, tmDU, a)
+                 : launch_scan<Sh>(scan_bwd_kernel<Sh, false, CL>, granted[0], groups, a.B, S, st, tmK, tmU, tmH, tmG, tmDK, tmDU, a);
 }
 
 }  // namespace grb
@@ -465,23 +645,13 @@ extern "C" int grb_scan_fwd(const void* k, const void* u, int64_t ldku, const fl
                             float* h_last, int B, int T, int C, int* err, void* stream) {
   if (B <= 0 || T <= 0 || C <= 0) return 0;
   if (C % 2) return -20;
-  CUtensorMap tmK, tmU, tmH;
-  int rc = make_tmap_btc_bf16(&tmK, k, C, T, B, ldku, SC_CH, F_TS);
-  if (rc) return rc;
-  rc = make_tmap_btc_bf16(&tmU, u, C, T, B, ldku, SC_CH, F_TS);
-  if (rc) return rc;
-  // the output leaves through bulk tensor stores when its layout allows a tensor map (16-byte aligned base and rows)
-  const bool tma_out = make_tmap_btc_bf16(&tmH, h, C, T, B, ldh, SC_CH, F_STEPS) == 0;
-  if (!tma_out) tmH = tmK;
-  static bool attr[2] = {false, false};
-  rc = tma_out ? allow_smem(scan_fwd_kernel<true>, F_SMEM, attr[1]) : allow_smem(scan_fwd_kernel<false>, F_SMEM, attr[0]);
-  if (rc) return rc;
-  ScanFwdArgs a{B, T, C, h0, reinterpret_cast<__nv_bfloat16*>(h), ldh, h_last, err};
-  dim3 grid((C + SC_CH - 1) / SC_CH, B);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (tma_out) scan_fwd_kernel<true><<<grid, SC_THREADS, F_SMEM, st>>>(tmK, tmU, tmH, a);
-  else scan_fwd_kernel<false><<<grid, SC_THREADS, F_SMEM, st>>>(tmK, tmU, tmH, a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  const ScanIo io{k, u, ldku};
+  const ScanFwdArgs a{B, T, C, h0, reinterpret_cast<__nv_bfloat16*>(h), ldh, h_last, err};
+  const int groups = (C + SC_CH - 1) / SC_CH * B;
+  const int S = pick_split<FwdC>(scan_fwd_kernel<FwdC, true, true>, groups, T);
+  if (S > 1 && T > S * FwdC::TS) return run_fwd<FwdC, true>(io, a, S, stream);
+  const int Ss = pick_split<FwdCShort>(scan_fwd_kernel<FwdCShort, true, true>, groups, T);
+  return Ss > 1 ? run_fwd<FwdCShort, true>(io, a, Ss, stream) : run_fwd<Fwd1, false>(io, a, 1, stream);
 }
 
 extern "C" int grb_scan_bwd(const void* k, const void* u, int64_t ldku, const void* h, int64_t ldh, const void* g,
@@ -489,25 +659,8 @@ extern "C" int grb_scan_bwd(const void* k, const void* u, int64_t ldku, const vo
                             float* dh0, const float* rowscale, int B, int T, int C, int* err, void* stream) {
   if (B <= 0 || T <= 0 || C <= 0) return 0;
   if (C % 2) return -20;
-  CUtensorMap tmK, tmU, tmH, tmG, tmDK, tmDU;
-  int rc = make_tmap_btc_bf16(&tmK, k, C, T, B, ldku, SC_CH, R_TS);
-  if (rc) return rc;
-  rc = make_tmap_btc_bf16(&tmU, u, C, T, B, ldku, SC_CH, R_TS);
-  if (rc) return rc;
-  rc = make_tmap_btc_bf16(&tmH, h, C, T, B, ldh, SC_CH, R_TS);
-  if (rc) return rc;
-  rc = make_tmap_btc_bf16(&tmG, g, C, T, B, ldg, SC_CH, R_TS);
-  if (rc) return rc;
-  const bool tma_out = make_tmap_btc_bf16(&tmDK, dk, C, T, B, ldd, SC_CH, R_STEPS) == 0 &&
-                       make_tmap_btc_bf16(&tmDU, du, C, T, B, ldd, SC_CH, R_STEPS) == 0;
-  if (!tma_out) tmDK = tmDU = tmK;
-  static bool attr[2] = {false, false};
-  rc = tma_out ? allow_smem(scan_bwd_kernel<true>, R_SMEM, attr[1]) : allow_smem(scan_bwd_kernel<false>, R_SMEM, attr[0]);
-  if (rc) return rc;
-  ScanBwdArgs a{B, T, C, h0, dh_last, reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(du), ldd, dh0, rowscale, err};
-  dim3 grid((C + SC_CH - 1) / SC_CH, B);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (tma_out) scan_bwd_kernel<true><<<grid, SC_THREADS, R_SMEM, st>>>(tmK, tmU, tmH, tmG, tmDK, tmDU, a);
-  else scan_bwd_kernel<false><<<grid, SC_THREADS, R_SMEM, st>>>(tmK, tmU, tmH, tmG, tmDK, tmDU, a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  const ScanIo io{k, u, ldku, h, ldh, g, ldg};
+  const ScanBwdArgs a{B, T, C, h0, dh_last, reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(du), ldd, dh0, rowscale, err};
+  const int S = pick_split<BwdC>(scan_bwd_kernel<BwdC, true, true>, (C + SC_CH - 1) / SC_CH * B, T);
+  return S > 1 ? run_bwd<BwdC, true>(io, a, S, stream) : run_bwd<Bwd1, false>(io, a, 1, stream);
 }
