@@ -167,233 +167,112 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const f
   }
 }
 
-// Faster variant for D <= 4096: a CTA of 256 threads walks groups of RB rows; thread t owns the float4 columns
-// t, t+256, ... of every row, so the dw / dcol partial sums stay in registers for the whole kernel and only the
-// per-row dot product needs a block reduction (one __syncthreads per group, double-buffered partials).
-template <int NCH>
-__global__ void __launch_bounds__(256, 2)
-rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const float* __restrict__ x,
-                        const float* __restrict__ rstd, const float* __restrict__ w,
-                        const float* __restrict__ dres_in, float* __restrict__ dres_out,
-                        __nv_bfloat16* __restrict__ dres16, float* __restrict__ dw, float* __restrict__ dcol,
-                        int64_t M, int D, int prescaled) {
-  constexpr int RB = NCH == 1 ? 4 : 2;
-  __shared__ float part[2][RB][8];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nv = D / 4;
-  float4 wv[NCH], adw[NCH], adc[NCH];
-  bool act[NCH];
+// D <= 4096: a group of G warps per row (D <= 1024 G), WARPS / G groups per CTA, each walking rows of its own.  A lane owns
+// the float4 columns lane, lane + 32 G, ... of every row, holds the row in registers between the dot product and the
+// update, and keeps the dw / dcol partial sums of its columns in registers for the whole kernel; with G = 1 a row needs no
+// barrier at all, otherwise one named barrier of the group.  Streaming bound (16 bytes per element): what keeps HBM busy is
+// a row (up to 40 KB) in flight per group, independent of the other groups.  One atomic per column and CTA at the end.
+template <int NV, int G, int WARPS, int MINB>
+__global__ void __launch_bounds__(32 * WARPS, MINB)
+rmsnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ dy, const float* __restrict__ x,
+                         const float* __restrict__ rstd, const float* __restrict__ w,
+                         const float* __restrict__ dres_in, float* __restrict__ dres_out,
+                         __nv_bfloat16* __restrict__ dres16, float* __restrict__ dw, float* __restrict__ dcol,
+                         int64_t M, int D, int prescaled) {
+  constexpr int GROUPS = WARPS / G;
+  extern __shared__ float4 sh[];                  // w [nv]; reused for the column sums at the end
+  __shared__ float part[GROUPS][2][G];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = warp / G, sub = warp % G;
+  const int nv = D / 4, i0 = sub * 32 + lane;
+  for (int i = threadIdx.x; i < nv; i += 32 * WARPS) sh[i] = reinterpret_cast<const float4*>(w)[i];
+  __syncthreads();
+  float4 adw[NV], adc[NV];
 #pragma unroll
-  for (int j = 0; j < NCH; ++j) {
-    act[j] = tid + 256 * j < nv;
-    wv[j] = act[j] ? reinterpret_cast<const float4*>(w)[tid + 256 * j] : make_float4(0, 0, 0, 0);
-    adw[j] = make_float4(0, 0, 0, 0);
-    adc[j] = make_float4(0, 0, 0, 0);
-  }
-  int buf = 0;
-  for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * RB; r0 < M; r0 += static_cast<int64_t>(gridDim.x) * RB, buf ^= 1) {
-    float4 xv[RB][NCH], pv[RB][NCH];      // x, incoming residual gradient (prefetched with the first loads)
-    uint2 dv[RB][NCH];
-    float dot[RB];
+  for (int j = 0; j < NV; ++j) adw[j] = adc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float inv_d = 1.f / D;
+  int par = 0;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * GROUPS;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * GROUPS + group; r < M; r += stride, par ^= 1) {
+    const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(r) * D);
+    const uint2* dyr = reinterpret_cast<const uint2*>(dy + static_cast<size_t>(r) * D);
+    const float4* pr = dres_in ? reinterpret_cast<const float4*>(dres_in + static_cast<size_t>(r) * D) : nullptr;
+    float4 xv[NV], pv[NV];
+    uint2 dv[NV];
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      const int64_t row = r0 + r;
-      dot[r] = 0.f;
-#pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        if (row < M && act[j]) {
-          xv[r][j] = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * D)[tid + 256 * j];
-          dv[r][j] = reinterpret_cast<const uint2*>(dy + static_cast<size_t>(row) * D)[tid + 256 * j];
-          pv[r][j] = dres_in ? reinterpret_cast<const float4*>(dres_in + static_cast<size_t>(row) * D)[tid + 256 * j]
-                             : make_float4(0, 0, 0, 0);
-        } else {
-          xv[r][j] = make_float4(0, 0, 0, 0);
-          pv[r][j] = make_float4(0, 0, 0, 0);
-          dv[r][j] = make_uint2(0, 0);
-        }
-        dot[r] += bf16_lo(dv[r][j].x) * wv[j].x * xv[r][j].x + bf16_hi(dv[r][j].x) * wv[j].y * xv[r][j].y +
-                  bf16_lo(dv[r][j].y) * wv[j].z * xv[r][j].z + bf16_hi(dv[r][j].y) * wv[j].w * xv[r][j].w;
-      }
+    for (int j = 0; j < NV; ++j) {
+      const int i = i0 + 32 * G * j;
+      const bool in = i < nv;
+      xv[j] = in ? xr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      dv[j] = in ? dyr[i] : make_uint2(0u, 0u);
+      pv[j] = in && pr ? pr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    const float rs = rstd[r];
+    float dot = 0.f;
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      const float s = warp_sum(dot[r]);
-      if (lane == 0) part[buf][r][warp] = s;
+    for (int j = 0; j < NV; ++j) {
+      const int i = i0 + 32 * G * j;
+      const float4 g = i < nv ? sh[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      dot += bf16_lo(dv[j].x) * g.x * xv[j].x + bf16_hi(dv[j].x) * g.y * xv[j].y + bf16_lo(dv[j].y) * g.z * xv[j].z +
+             bf16_hi(dv[j].y) * g.w * xv[j].w;
     }
-    __syncthreads();
+    dot = warp_sum(dot);
+    if constexpr (G > 1) {
+      if (lane == 0) part[group][par][sub] = dot;
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * G) : "memory");
+      dot = 0.f;
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      const int64_t row = r0 + r;
-      if (row >= M) break;
-      float tot = 0.f;
+      for (int k = 0; k < G; ++k) dot += part[group][par][k];
+    }
+    const float so = prescaled ? 1.f : rs;
+    const float sx = so * rs * rs * dot * inv_d;
+    float4* dro = reinterpret_cast<float4*>(dres_out + static_cast<size_t>(r) * D);
+    uint2* dr16 = dres16 ? reinterpret_cast<uint2*>(dres16 + static_cast<size_t>(r) * D) : nullptr;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) tot += part[buf][r][k];
-      const float rs = rstd[row];
-      const float so = prescaled ? 1.f : rs;
-      const float sx = so * rs * rs * tot / D;
-#pragma unroll
-      for (int j = 0; j < NCH; ++j) {
-        if (!act[j]) continue;
-        const size_t off = static_cast<size_t>(row) * D / 4 + tid + 256 * j;
-        const float d0 = bf16_lo(dv[r][j].x), d1 = bf16_hi(dv[r][j].x), d2 = bf16_lo(dv[r][j].y), d3 = bf16_hi(dv[r][j].y);
-        const float h0 = xv[r][j].x * so, h1 = xv[r][j].y * so, h2 = xv[r][j].z * so, h3 = xv[r][j].w * so;
+    for (int j = 0; j < NV; ++j) {
+      const int i = i0 + 32 * G * j;
+      if (i < nv) {
+        const float4 g = sh[i];
+        const float d0 = so * bf16_lo(dv[j].x), d1 = so * bf16_hi(dv[j].x), d2 = so * bf16_lo(dv[j].y), d3 = so * bf16_hi(dv[j].y);
         float4 o;
-        o.x = so * d0 * wv[j].x - xv[r][j].x * sx;
-        o.y = so * d1 * wv[j].y - xv[r][j].y * sx;
-        o.z = so * d2 * wv[j].z - xv[r][j].z * sx;
-        o.w = so * d3 * wv[j].w - xv[r][j].w * sx;
-        o.x += pv[r][j].x; o.y += pv[r][j].y; o.z += pv[r][j].z; o.w += pv[r][j].w;
-        reinterpret_cast<float4*>(dres_out)[off] = o;
-        if (dres16) reinterpret_cast<uint2*>(dres16)[off] = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
-        adw[j].x += d0 * h0; adw[j].y += d1 * h1; adw[j].z += d2 * h2; adw[j].w += d3 * h3;
+        o.x = fmaf(d0, g.x, fmaf(-xv[j].x, sx, pv[j].x));
+        o.y = fmaf(d1, g.y, fmaf(-xv[j].y, sx, pv[j].y));
+        o.z = fmaf(d2, g.z, fmaf(-xv[j].z, sx, pv[j].z));
+        o.w = fmaf(d3, g.w, fmaf(-xv[j].w, sx, pv[j].w));
+        dro[i] = o;
+        if (dr16) dr16[i] = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
+        adw[j].x = fmaf(d0, xv[j].x, adw[j].x); adw[j].y = fmaf(d1, xv[j].y, adw[j].y);
+        adw[j].z = fmaf(d2, xv[j].z, adw[j].z); adw[j].w = fmaf(d3, xv[j].w, adw[j].w);
         adc[j].x += o.x; adc[j].y += o.y; adc[j].z += o.z; adc[j].w += o.w;
       }
     }
   }
+  // column sums of the CTA: the groups add into shared memory one after the other, then one reduction per four columns
+  for (int pass = 0; pass < (dcol ? 2 : 1); ++pass) {
+    for (int q = 0; q < GROUPS; ++q) {
+      __syncthreads();
+      if (q == group) {
 #pragma unroll
-  for (int j = 0; j < NCH; ++j) {
-    if (!act[j]) continue;
-    const int c0 = 4 * (tid + 256 * j);
-    atomicAdd(dw + c0, adw[j].x); atomicAdd(dw + c0 + 1, adw[j].y); atomicAdd(dw + c0 + 2, adw[j].z); atomicAdd(dw + c0 + 3, adw[j].w);
-    if (dcol) {
-      atomicAdd(dcol + c0, adc[j].x); atomicAdd(dcol + c0 + 1, adc[j].y); atomicAdd(dcol + c0 + 2, adc[j].z); atomicAdd(dcol + c0 + 3, adc[j].w);
-    }
-  }
-}
-
-// Variant of the above whose inputs arrive through a ring of row slots in shared memory, filled by bulk copies
-// (cp.async.bulk, one mbarrier per slot): the bytes in flight per SM are the ring (up to 8 rows: 8 x 20 KB for D = 2048)
-// instead of what two CTAs can hold in registers, which is what a streaming kernel of 32 KB per row needs to keep
-// HBM busy.  Two CTAs per SM walk rows blockIdx.x, blockIdx.x + gridDim.x, ...; per row there is one mbarrier
-// wait and one __syncthreads (the block reduction of the row's dot product), after which every thread holds its
-// part of the row in registers and the slot is refilled.  Same results as rmsnorm_bwd_rows_kernel.
-constexpr int RING_MAX_SLOTS = 8;
-
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(smem_dst)),
-               "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-template <int NCH>
-__global__ void __launch_bounds__(256, 2)
-rmsnorm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const float* __restrict__ x,
-                        const float* __restrict__ rstd, const float* __restrict__ w,
-                        const float* __restrict__ dres_in, float* __restrict__ dres_out,
-                        __nv_bfloat16* __restrict__ dres16, float* __restrict__ dw, float* __restrict__ dcol,
-                        int64_t M, int D, int slots, int* err, int prescaled) {
-  extern __shared__ __align__(128) uint8_t ring[];
-  __shared__ uint64_t full[RING_MAX_SLOTS];
-  __shared__ float part[2][8];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nv = D / 4;
-  const uint32_t xb = D * 4, yb = D * 2;
-  const uint32_t slot_bytes = xb + (dres_in ? xb : 0) + yb;     // x | dres_in | dy, all multiples of 16 bytes
-  const int64_t first = blockIdx.x, stride = gridDim.x;
-  const int64_t nrows = first < M ? (M - first + stride - 1) / stride : 0;
-
-  if (tid == 0) {
-    for (int i = 0; i < RING_MAX_SLOTS; ++i) mbar_init(&full[i], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  auto issue = [&](int64_t i) {                                  // thread 0: start the copies of this CTA's i-th row
-    const int64_t row = first + i * stride;
-    uint8_t* dst = ring + static_cast<size_t>(i % slots) * slot_bytes;
-    uint64_t* bar = &full[i % slots];
-    mbar_expect_tx(bar, slot_bytes);
-    bulk_load(dst, x + row * D, xb, bar);
-    if (dres_in) bulk_load(dst + xb, dres_in + row * D, xb, bar);
-    bulk_load(dst + slot_bytes - yb, dy + row * D, yb, bar);
-  };
-  if (tid == 0)
-    for (int64_t i = 0; i < nrows && i < slots; ++i) issue(i);
-
-  float4 wv[NCH], adw[NCH], adc[NCH];
-  bool act[NCH];
-#pragma unroll
-  for (int j = 0; j < NCH; ++j) {
-    act[j] = tid + 256 * j < nv;
-    wv[j] = act[j] ? reinterpret_cast<const float4*>(w)[tid + 256 * j] : make_float4(0, 0, 0, 0);
-    adw[j] = make_float4(0, 0, 0, 0);
-    adc[j] = make_float4(0, 0, 0, 0);
-  }
-  float rs_next = nrows > 0 ? rstd[first] : 0.f;
-  bool ok = true;
-  int64_t done = 0;
-  for (int64_t i = 0; i < nrows; ++i) {
-    const int slot = static_cast<int>(i % slots);
-    const int64_t row = first + i * stride;
-    const float rs = rs_next;
-    if (i + 1 < nrows) rs_next = rstd[row + stride];
-    if (!mbar_wait(&full[slot], static_cast<uint32_t>((i / slots) & 1))) ok = false;
-    if (!__syncthreads_and(ok)) { ok = false; break; }          // block-uniform
-    done = i + 1;
-    const uint8_t* src = ring + static_cast<size_t>(slot) * slot_bytes;
-    float4 xv[NCH], pv[NCH];
-    uint2 dv[NCH];
-    float dot = 0.f;
-#pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-      if (act[j]) {
-        xv[j] = reinterpret_cast<const float4*>(src)[tid + 256 * j];
-        pv[j] = dres_in ? reinterpret_cast<const float4*>(src + xb)[tid + 256 * j] : make_float4(0, 0, 0, 0);
-        dv[j] = reinterpret_cast<const uint2*>(src + slot_bytes - yb)[tid + 256 * j];
-      } else {
-        xv[j] = make_float4(0, 0, 0, 0);
-        pv[j] = make_float4(0, 0, 0, 0);
-        dv[j] = make_uint2(0, 0);
+        for (int j = 0; j < NV; ++j) {
+          const int i = i0 + 32 * G * j;
+          if (i < nv) {
+            float4 v = pass ? adc[j] : adw[j];
+            if (q) { const float4 u = sh[i]; v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w; }
+            sh[i] = v;
+          }
+        }
       }
-      dot += bf16_lo(dv[j].x) * wv[j].x * xv[j].x + bf16_hi(dv[j].x) * wv[j].y * xv[j].y +
-             bf16_lo(dv[j].y) * wv[j].z * xv[j].z + bf16_hi(dv[j].y) * wv[j].w * xv[j].w;
     }
-    const float sdot = warp_sum(dot);
-    if (lane == 0) part[i & 1][warp] = sdot;
-    __syncthreads();                                            // partial sums visible; every thread has read the slot
-    if (tid == 0 && i + slots < nrows) {
-      fence_proxy_async_smem();                                 // those reads before the copy that overwrites the slot
-      issue(i + slots);
-    }
-    float tot = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) tot += part[i & 1][k];
-    const float so = prescaled ? 1.f : rs;
-    const float sx = so * rs * rs * tot / D;
-#pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-      if (!act[j]) continue;
-      const size_t off = static_cast<size_t>(row) * D / 4 + tid + 256 * j;
-      const float d0 = bf16_lo(dv[j].x), d1 = bf16_hi(dv[j].x), d2 = bf16_lo(dv[j].y), d3 = bf16_hi(dv[j].y);
-      const float h0 = xv[j].x * so, h1 = xv[j].y * so, h2 = xv[j].z * so, h3 = xv[j].w * so;
-      float4 o;
-      o.x = so * d0 * wv[j].x - xv[j].x * sx + pv[j].x;
-      o.y = so * d1 * wv[j].y - xv[j].y * sx + pv[j].y;
-      o.z = so * d2 * wv[j].z - xv[j].z * sx + pv[j].z;
-      o.w = so * d3 * wv[j].w - xv[j].w * sx + pv[j].w;
-      reinterpret_cast<float4*>(dres_out)[off] = o;
-      if (dres16) reinterpret_cast<uint2*>(dres16)[off] = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
-      adw[j].x += d0 * h0; adw[j].y += d1 * h1; adw[j].z += d2 * h2; adw[j].w += d3 * h3;
-      adc[j].x += o.x; adc[j].y += o.y; adc[j].z += o.z; adc[j].w += o.w;
-    }
-  }
-  if (!ok) {
-    // a copy did not arrive in time: report; give the copies still outstanding one more bounded wait each so that
-    // nothing lands in shared memory after the CTA has gone; the column sums of this CTA are dropped
-    if (tid == 0) {
-      atomicExch(err, 11);
-      const int64_t issued = nrows < done + slots ? nrows : done + slots;
-      for (int64_t i = done; i < issued; ++i) mbar_wait(&full[i % slots], static_cast<uint32_t>((i / slots) & 1));
-    }
-    return;
-  }
-#pragma unroll
-  for (int j = 0; j < NCH; ++j) {
-    if (!act[j]) continue;
-    const int c0 = 4 * (tid + 256 * j);
-    atomicAdd(dw + c0, adw[j].x); atomicAdd(dw + c0 + 1, adw[j].y); atomicAdd(dw + c0 + 2, adw[j].z); atomicAdd(dw + c0 + 3, adw[j].w);
-    if (dcol) {
-      atomicAdd(dcol + c0, adc[j].x); atomicAdd(dcol + c0 + 1, adc[j].y); atomicAdd(dcol + c0 + 2, adc[j].z); atomicAdd(dcol + c0 + 3, adc[j].w);
+    __syncthreads();
+    float* out = pass ? dcol : dw;
+    const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    for (int i = threadIdx.x; i < nv; i += 32 * WARPS) {
+      const float4 v = sh[i];
+      if (vec) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + 4 * i), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+      } else {
+        atomicAdd(out + 4 * i, v.x); atomicAdd(out + 4 * i + 1, v.y); atomicAdd(out + 4 * i + 2, v.z); atomicAdd(out + 4 * i + 3, v.w);
+      }
     }
   }
 }
@@ -508,61 +387,34 @@ extern "C" int grb_rmsnorm_fwd(const float* x, const float* w, void* y, float* r
   return LAUNCH_OK();
 }
 
-template <int NCH>
-static int launch_rmsnorm_ring(const __nv_bfloat16* dy, const float* x, const float* rstd, const float* w,
-                               const float* dres_in, float* dres_out, __nv_bfloat16* d16, float* dw, float* dcol, int64_t M,
-                               int D, int* err, int prescaled, cudaStream_t st) {
-  const size_t slot = static_cast<size_t>(D) * (dres_in ? 10 : 6);
-  // two CTAs per SM: while one waits at its per-row block barrier the other computes (with a single CTA the two
-  // barriers per row serialise the rows and the ring is slower than the register version)
-  constexpr int kCtasPerSm = 2;
-  int slots = static_cast<int>((200 * 1024 / kCtasPerSm) / slot);
-  if (slots > RING_MAX_SLOTS) slots = RING_MAX_SLOTS;
-  if (slots < 2) return -31;
-  const size_t smem = slot * slots;
-  static size_t granted = 0;
-  if (smem > 40 * 1024 && smem > granted) {
-    if (cudaFuncSetAttribute(rmsnorm_bwd_ring_kernel<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-        cudaSuccess)
-      return -4;
-    granted = smem;
-  }
-  const int blocks = static_cast<int>(std::min<int64_t>(M, static_cast<int64_t>(num_sms()) * kCtasPerSm));
-  rmsnorm_bwd_ring_kernel<NCH><<<blocks, 256, smem, st>>>(dy, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, slots, err,
-                                                          prescaled);
+template <int NV, int G, int WARPS, int MINB>
+static int launch_rmsnorm_group(const void* dy, const float* x, const float* rstd, const float* w, const float* dres_in,
+                                float* dres_out, void* dres16, float* dw, float* dcol, int64_t M, int D, int prescaled, void* st) {
+  constexpr int groups = WARPS / G;
+  const int blocks = static_cast<int>(std::min<int64_t>((M + groups - 1) / groups, static_cast<int64_t>(num_sms()) * MINB));
+  rmsnorm_bwd_group_kernel<NV, G, WARPS, MINB><<<blocks, 32 * WARPS, D * sizeof(float), ST(st)>>>(
+      reinterpret_cast<const __nv_bfloat16*>(dy), x, rstd, w, dres_in, dres_out, reinterpret_cast<__nv_bfloat16*>(dres16), dw,
+      dcol, M, D, prescaled);
   return LAUNCH_OK();
 }
 
 extern "C" int grb_rmsnorm_bwd(const void* dy, const float* x, const float* rstd, const float* w, const float* dres_in,
                                float* dres_out, void* dres16, float* dw, float* dcol, int64_t M, int D, int prescaled,
-                               int* err, void* stream) {
+                               void* stream) {
   if (D % 4) return -30;
   if (M == 0) return 0;
-  // shared-memory ring fed by bulk copies: needs 16-byte rows in every input and a ring that fits
-  const bool aligned = D % 8 == 0 && !((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) |
-                                        reinterpret_cast<uintptr_t>(dres_in)) & 15);
-  if (err && aligned && D <= 3072 && M >= 4 * num_sms()) {      // (wider rows need more registers than two CTAs per SM leave)
-    const __nv_bfloat16* dyp = reinterpret_cast<const __nv_bfloat16*>(dy);
-    __nv_bfloat16* d16 = reinterpret_cast<__nv_bfloat16*>(dres16);
-    switch ((D / 4 + 255) / 256) {
-      case 1: return launch_rmsnorm_ring<1>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, err, prescaled, ST(stream));
-      case 2: return launch_rmsnorm_ring<2>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, err, prescaled, ST(stream));
-      default: return launch_rmsnorm_ring<3>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, err, prescaled, ST(stream));
-    }
-  }
-  if (D <= 4096) {
-    const int nch = (D / 4 + 255) / 256;
-    const int blocks = static_cast<int>(std::min<int64_t>((M + 1) / 2, num_sms() * 4));
-    const __nv_bfloat16* dyp = reinterpret_cast<const __nv_bfloat16*>(dy);
-    __nv_bfloat16* d16 = reinterpret_cast<__nv_bfloat16*>(dres16);
-    switch (nch) {
-      case 1: rmsnorm_bwd_rows_kernel<1><<<blocks, 256, 0, ST(stream)>>>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, prescaled); break;
-      case 2: rmsnorm_bwd_rows_kernel<2><<<blocks, 256, 0, ST(stream)>>>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, prescaled); break;
-      case 3: rmsnorm_bwd_rows_kernel<3><<<blocks, 256, 0, ST(stream)>>>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, prescaled); break;
-      default: rmsnorm_bwd_rows_kernel<4><<<blocks, 256, 0, ST(stream)>>>(dyp, x, rstd, w, dres_in, dres_out, d16, dw, dcol, M, D, prescaled); break;
-    }
-    return LAUNCH_OK();
-  }
+  // four float4 columns per lane: more (fewer warps per row) leaves one CTA per SM, too few rows in flight.  M x D, 16 bytes per
+  // element: 8188 x 512 16 us (one block of 256 threads per row: 40), 2047 x 1024 9.7 (22), 16376 x 2048 91 (93),
+  // 4000 x 4096 44 (104).
+#define GRB_NORM(NV, G, WARPS, MINB) \
+  return launch_rmsnorm_group<NV, G, WARPS, MINB>(dy, x, rstd, w, dres_in, dres_out, dres16, dw, dcol, M, D, prescaled, stream)
+  if (D <= 256) GRB_NORM(2, 1, 8, 3);
+  if (D <= 512) GRB_NORM(4, 1, 8, 2);
+  if (D <= 1024) GRB_NORM(4, 2, 8, 2);
+  if (D <= 2048) GRB_NORM(4, 4, 8, 2);
+  if (D <= 3072) GRB_NORM(4, 6, 12, 1);
+  if (D <= 4096) GRB_NORM(4, 8, 16, 1);
+#undef GRB_NORM
   int warps = 8;
   while (warps > 1 && static_cast<size_t>(2 * warps) * D * sizeof(float) > 160 * 1024) warps >>= 1;
   const size_t smem = static_cast<size_t>(2 * warps) * D * sizeof(float);

@@ -238,11 +238,12 @@ def decode_tc(mode: int, src, w16, out, *, vec=None, state=None, state_out=None,
 
 def rmsnorm_bwd(dy16, x, rstd, w, dres_in, dres_out, dres16, dw, dcol=None, ring=True, prescaled=False):
     """RMSNorm backward fused with the residual-gradient accumulation (``csrc/elementwise.cu``).  ``prescaled``:
-    ``dy16`` is the gradient w.r.t. the unnormalised x * w (the norm was folded into its consumer GEMM)."""
+    ``dy16`` is the gradient w.r.t. the unnormalised x * w (the norm was folded into its consumer GEMM).  ``ring`` is
+    accepted and has no effect (it chose between two kernels where there is one)."""
     M, D = x.shape
     L.check(L.lib().grb_rmsnorm_bwd(dy16.data_ptr(), x.data_ptr(), rstd.data_ptr(), w.data_ptr(), L.ptr(dres_in),
                                     dres_out.data_ptr(), L.ptr(dres16), dw.data_ptr(), L.ptr(dcol), M, D, int(prescaled),
-                                    L.err_flag(x.device).data_ptr() if ring else None, L.stream()),
+                                    L.stream()),
             "grb_rmsnorm_bwd")
     _count()
 

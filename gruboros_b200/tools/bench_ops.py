@@ -5,7 +5,7 @@
             autocast; mingru/minGRU.py:16-28,56-67) and vs. the HBM roofline.
   gemm      the tcgen05 GEMMs on the 1B model's shapes vs. torch.matmul (cuBLAS).
   gemm_fused the fused-epilogue GEMMs exactly as a 1B layer issues them (residual add, bias + GELU, GELU').
-  rmsnorm   RMSNorm backward (+ residual-gradient accumulation): shared-memory ring vs. register version.
+  rmsnorm   RMSNorm backward (+ residual-gradient accumulation).
   optimizer fused Schedule-Free AdamW vs. the HBM roofline.
 
     python -m gruboros_b200.tools.bench_ops [scan] [gemm] [gemm_fused] [rmsnorm] [optimizer]   -> one JSON object on stdout
@@ -288,14 +288,12 @@ def bench_rmsnorm(M=16376, D=2048):
 
     nbytes = M * D * 16.0
     res = {"rows": M, "dim": D}
-    for name, ring in (("shared_memory_ring", True), ("register_rows", False)):
-        def run():
-            i = next(it) % n_buf
-            K.rmsnorm_bwd(dys[i], xs[i], rstd, w, ds[i], out, o16, dw, dc, ring=ring)
+    def run():
+        i = next(it) % n_buf
+        K.rmsnorm_bwd(dys[i], xs[i], rstd, w, ds[i], out, o16, dw, dc)
 
-        t = timeit(run, iters=18)
-        res[name] = {"us": round(t * 1e3, 1), "GBs": round(nbytes / t / 1e6, 1),
-                     "frac_of_%s_hbm" % src: round(nbytes / t / 1e6 / hbm, 3)}
+    t = timeit(run, iters=18)
+    res.update({"us": round(t * 1e3, 1), "GBs": round(nbytes / t / 1e6, 1), "frac_of_%s_hbm" % src: round(nbytes / t / 1e6 / hbm, 3)})
     return res
 
 
