@@ -8,9 +8,6 @@
 #include <cuda_runtime.h>
 #include <mutex>
 
-extern "C" int grb_gemm_pair(int major_a, int major_b, int epi, const void* A, int64_t lda, const void* B, int64_t ldb,
-                             int M, int N, int K, int splitk, const EpiArgs* e, int* err, int max_ctas, void* stream);
-
 namespace {
 
 // Per-row losses of the call in flight.  In host code this name is only a handle for the runtime, not a device
@@ -48,11 +45,7 @@ extern "C" int grb_ce_loss_static(const void* x16, int64_t ldx, const void* w16,
   e.aux = labels;
   e.ldo = dlogits ? ldd : V;
   e.alpha = grad_scale;
-  // same kernel choice as the regular path: CTA pairs once there are enough 256-row tiles to fill the machine
-  const int pair_tiles = (M + 255) / 256;
-  const int rc = pair_tiles >= 48
-                     ? grb_gemm_pair(MAJOR_K, MAJOR_K, EPI_CE, x16, ldx, w16, ldw, M, V, K, 1, &e, err, 0, stream)
-                     : grb_gemm(MAJOR_K, MAJOR_K, EPI_CE, x16, ldx, w16, ldw, M, V, K, 1, &e, err, 0, stream);
+  const int rc = grb_gemm(MAJOR_K, MAJOR_K, EPI_CE, x16, ldx, w16, ldw, M, V, K, 1, &e, err, 0, stream);
   if (rc) return rc;
   return grb_sum_scale(rows, M, loss_scale_out, loss_out, 0, stream);
 }

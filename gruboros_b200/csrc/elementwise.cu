@@ -7,6 +7,7 @@
 // (mingru/minLM.py:67-74,120,130,137) and the autograd of both.
 #include "ptx.cuh"
 #include "elementwise.h"
+#include "launch.h"
 #include <algorithm>
 
 namespace grb {
@@ -29,6 +30,8 @@ __global__ void embed_fwd_kernel(const uint8_t* __restrict__ tokens, int64_t str
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t M = static_cast<int64_t>(B) * T;
+  pdl_trigger();
+  pdl_wait();
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * warps_per_block + warp; r < M;
        r += static_cast<int64_t>(gridDim.x) * warps_per_block) {
     const int b = static_cast<int>(r / T), t = static_cast<int>(r % T);
@@ -185,6 +188,8 @@ rmsnorm_bwd_group_kernel(const __nv_bfloat16* __restrict__ dy, const float* __re
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = warp / G, sub = warp % G;
   const int nv = D / 4, i0 = sub * 32 + lane;
+  pdl_trigger();
+  pdl_wait();
   for (int i = threadIdx.x; i < nv; i += 32 * WARPS) sh[i] = reinterpret_cast<const float4*>(w)[i];
   __syncthreads();
   float4 adw[NV], adc[NV];
@@ -308,6 +313,8 @@ __global__ void sum_scale_kernel(const float* __restrict__ v, int64_t n, float s
                                  int accumulate) {
   __shared__ float red[32];
   float s = 0.f;
+  pdl_trigger();
+  pdl_wait();
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -372,10 +379,8 @@ extern "C" int grb_embed_fwd(const uint8_t* tokens, int64_t stride, int B, int T
   if (M == 0) return 0;
   const int blocks = static_cast<int>(std::min<int64_t>((M + 7) / 8, num_sms() * 8));
   if (normw && (!xw || !ssq || parts < 1)) return -32;
-  embed_fwd_kernel<<<blocks, 256, 0, ST(stream)>>>(tokens, stride, B, T, D, V, E, x, labels,
-                                                  reinterpret_cast<__nv_bfloat16*>(onehot), normw,
-                                                  reinterpret_cast<__nv_bfloat16*>(xw), ssq, parts);
-  return LAUNCH_OK();
+  return launch_pdl(embed_fwd_kernel, dim3(blocks), 256, 0, ST(stream), 1, tokens, stride, B, T, D, V, E, x, labels,
+                    reinterpret_cast<__nv_bfloat16*>(onehot), normw, reinterpret_cast<__nv_bfloat16*>(xw), ssq, parts);
 }
 
 extern "C" int grb_rmsnorm_fwd(const float* x, const float* w, void* y, float* rstd, int64_t M, int D, float eps,
@@ -392,10 +397,9 @@ static int launch_rmsnorm_group(const void* dy, const float* x, const float* rst
                                 float* dres_out, void* dres16, float* dw, float* dcol, int64_t M, int D, int prescaled, void* st) {
   constexpr int groups = WARPS / G;
   const int blocks = static_cast<int>(std::min<int64_t>((M + groups - 1) / groups, static_cast<int64_t>(num_sms()) * MINB));
-  rmsnorm_bwd_group_kernel<NV, G, WARPS, MINB><<<blocks, 32 * WARPS, D * sizeof(float), ST(st)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(dy), x, rstd, w, dres_in, dres_out, reinterpret_cast<__nv_bfloat16*>(dres16), dw,
-      dcol, M, D, prescaled);
-  return LAUNCH_OK();
+  return launch_pdl(rmsnorm_bwd_group_kernel<NV, G, WARPS, MINB>, dim3(blocks), 32 * WARPS, D * sizeof(float), ST(st), 1,
+                    reinterpret_cast<const __nv_bfloat16*>(dy), x, rstd, w, dres_in, dres_out,
+                    reinterpret_cast<__nv_bfloat16*>(dres16), dw, dcol, M, D, prescaled);
 }
 
 extern "C" int grb_rmsnorm_bwd(const void* dy, const float* x, const float* rstd, const float* w, const float* dres_in,
@@ -442,8 +446,7 @@ extern "C" int grb_colsum_bf16(const void* a, int64_t ld, int64_t M, int N, floa
 }
 
 extern "C" int grb_sum_scale(const float* v, int64_t n, float scale, float* out, int accumulate, void* stream) {
-  sum_scale_kernel<<<1, 1024, 0, ST(stream)>>>(v, n, scale, out, accumulate);
-  return LAUNCH_OK();
+  return launch_pdl(sum_scale_kernel, dim3(1), 1024, 0, ST(stream), 1, v, n, scale, out, accumulate);
 }
 
 extern "C" int grb_cast_f32_bf16(const float* in, void* out, int64_t n, void* stream) {

@@ -1,19 +1,17 @@
-// Fused GEMM epilogues shared by the one-CTA and the CTA-pair tcgen05 kernels.
+// Fused GEMM epilogues of the tcgen05 kernels: the math of four neighbouring columns (epilogue_apply4, both kernels) and
+// the CTA-pair kernel's warp loops.
 //
 // tcgen05.ld hands each thread one accumulator ROW (TMEM lane) x 32 columns.  Writing that straight to global
 // memory makes every warp store touch 32 different cache lines, 16 bytes each, and the L1-to-crossbar request
 // rate - not the tensor pipe - ends up limiting the kernel.  So each warp first transposes its 32 x 32 chunk
 // through a private shared-memory staging tile; afterwards a lane owns 4 consecutive columns of a row, 8 lanes
 // cover a 128-byte row segment and every load / store / reduction instruction moves whole cache lines.
-// The cross-entropy epilogue keeps the row-per-thread form (it needs whole rows and writes little).
 #pragma once
 #include "ptx.cuh"
 #include "owner.cuh"
 #include "gemm_sm100.h"
 
 namespace grb {
-
-constexpr int EPI_BN = 256;   // accumulator columns per tile
 
 // Checked build (-DGRB_CHECKS): `cond` is what an access about to be made relies on.  When it does not hold, the
 // code is recorded in the launch's error word and the caller skips the access - nothing traps, the kernel runs to
@@ -91,81 +89,6 @@ constexpr int EPI_STAGE_LD = 32;                         // floats per staged ro
                                                          // (conflict-free for the row-per-lane writes and the 8-lanes-per-row reads)
 constexpr int EPI_STAGE_FLOATS = 32 * EPI_STAGE_LD;      // per warp
 constexpr int EPI_STAGE_BYTES = EPI_STAGE_FLOATS * 4;
-
-// ------------------------------------------------------------- cross-entropy (row per thread)
-template <int EPI>
-__device__ __forceinline__ void epilogue_row(const EpiArgs& e, uint32_t taddr, int row, int n0, int M, int N,
-                                             int c_begin, int c_end) {
-  const bool row_ok = row < M;
-  if constexpr (EPI == EPI_CE) {
-    // 256-way softmax cross-entropy on the accumulator row, v = rowscale * acc.
-    // loss_rows[row] = logsumexp(v) - v[label];  dlogits = (softmax - onehot) * alpha * rowscale
-    float* loss_rows = reinterpret_cast<float*>(e.out1);
-    __nv_bfloat16* dlog = reinterpret_cast<__nv_bfloat16*>(e.out0);
-    const uint8_t* labels = reinterpret_cast<const uint8_t*>(e.aux);
-    const int label = row_ok ? static_cast<int>(labels[row]) : 0;
-    const float rs = row_scale(e, row, M);     // logits = rs * accumulator (final RMSNorm folded in)
-    if (e.rstd_out && row_ok) e.rstd_out[row] = rs;
-    const float dscale = e.alpha * rs;         // ... and d logits carry rs too: the gradient w.r.t. the unnormalised operand
-    float mx = -INFINITY;
-    uint32_t r[32];
-    for (int c = 0; c < EPI_BN; c += 32) {
-      if (n0 + c >= N) break;
-      __syncwarp();
-      tmem_ld32(taddr + c, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (n0 + c + j < N) mx = fmaxf(mx, rs * __uint_as_float(r[j]));
-    }
-    float sum = 0.f, picked = 0.f;
-    for (int c = 0; c < EPI_BN; c += 32) {
-      if (n0 + c >= N) break;
-      __syncwarp();
-      tmem_ld32(taddr + c, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float v = rs * __uint_as_float(r[j]);
-        if (n0 + c + j < N) {
-          sum += __expf(v - mx);
-          if (n0 + c + j == label) picked = v;
-        }
-      }
-    }
-    const float lse = mx + __logf(sum);
-    if (row_ok && loss_rows) loss_rows[row] = lse - picked;
-    if (dlog) {
-      for (int c = 0; c < EPI_BN; c += 32) {
-        if (n0 + c >= N) break;
-        __syncwarp();
-        tmem_ld32(taddr + c, r);
-        tmem_ld_wait();
-        if (row_ok) {
-          __nv_bfloat16* dst = dlog + static_cast<size_t>(row) * e.ldo + n0 + c;
-          if (n0 + c + 32 <= N) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              float p0 = __expf(rs * __uint_as_float(r[j]) - lse) - ((n0 + c + j) == label ? 1.f : 0.f);
-              float p1 = __expf(rs * __uint_as_float(r[j + 1]) - lse) - ((n0 + c + j + 1) == label ? 1.f : 0.f);
-              pk[j >> 1] = pack_bf16(p0 * dscale, p1 * dscale);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              reinterpret_cast<uint4*>(dst)[j] = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
-          } else {
-            for (int j = 0; j < 32 && n0 + c + j < N; ++j) {
-              float p = __expf(rs * __uint_as_float(r[j]) - lse) - ((n0 + c + j) == label ? 1.f : 0.f);
-              dst[j] = __float2bfloat16(p * dscale);
-            }
-          }
-        }
-      }
-    }
-    return;
-  }
-}
 
 // ------------------------------------------------------------- element-wise epilogues (staged, coalesced)
 // One call handles 4 consecutive columns (col .. col+3) of one row.  `n_ok` = how many of them are inside N.

@@ -26,6 +26,7 @@
 #include "ptx.cuh"
 #include "gemm_sm100.h"
 #include "tmap.h"
+#include "launch.h"
 #include "gemm_epilogue.cuh"
 #include <cstdio>
 
@@ -231,6 +232,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_sync_all();          // barriers of both CTAs are initialised, tensor memory is allocated
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  if (warp != 1) pdl_wait();   // (the MMA warp touches no global memory)
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer (both CTAs)
@@ -320,8 +323,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ---------------------------------------------------------- epilogue (both CTAs)
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
-    const int c_begin = (EPI == EPI_CE) ? 0 : half * (BN / 2);
-    const int c_end = (EPI == EPI_CE) ? (half == 0 ? BN : 0) : (half + 1) * (BN / 2);
+    const int c_begin = half * (BN / 2), c_end = c_begin + BN / 2;
     int acc = 0; uint32_t accphase = 0; bool ok = true;
     WorkIter it = make_work(s.M, s.N, s.K, s.splitk, pair_id, npairs);
     Work w;
@@ -330,12 +332,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait(&tfull[acc], accphase)) { ok = false; break; }
       tc_fence_after();
       const bool tile_ok = grb_ok(e, tm >= 0 && tm < it.ntm && tn >= 0 && tn < it.ntn && w.kb0 >= 0 && w.kb1 <= it.nkb, GRB_CHK_TILE);
-      if (tile_ok && w.kb1 > w.kb0 && c_end > c_begin) {
+      if (tile_ok && w.kb1 > w.kb0) {
         const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
         const int row0 = tm * 2 * BM + static_cast<int>(rank) * BM + q * 32;
-        if constexpr (EPI == EPI_CE)
-          epilogue_row<EPI>(e, taddr, row0 + lane, tn * BN, s.M, s.N, c_begin, c_end);
-        else if constexpr (EPI == EPI_STORE_BF16 && GRB_TMA_STORE)
+        if constexpr (EPI == EPI_STORE_BF16 && GRB_TMA_STORE)
           epilogue_tma_store_bf16(e, &tmC, taddr, row0, tn * BN, s.M, s.N, c_begin, c_end,
                                   reinterpret_cast<uint8_t*>(epi_stage) + (warp - 2) * 4096, lane);
         else
@@ -402,16 +402,7 @@ static int launch(const void* A, int64_t lda, const void* B, int64_t ldb, int M,
   Shape s{M, N, K, splitk, err};
   EpiArgs ec = e;
   ec.chk_err = err;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, s, ec) == cudaSuccess ? 0 : -5;
+  return launch_pdl(kern, dim3(2 * pairs), NUM_THREADS, SMEM_BYTES, st, 2, tmA, tmB, tmC, s, ec);
 }
 
 }  // namespace pair
@@ -423,7 +414,6 @@ extern "C" int grb_gemm_pair(int major_a, int major_b, int epi, const void* A, i
                              int M, int N, int K, int splitk, const EpiArgs* e, int* err, int max_ctas, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (epi != EPI_RED_F32 && epi != EPI_RED_SCATTER && (splitk > 1 || splitk < 0)) return -10;
-  if (epi == EPI_CE && N > pair::BN) return -11;
 #define GRB_CASE(MA, MB, EP)                                                   \
   if (major_a == MA && major_b == MB && epi == EP)                             \
     return pair::launch<MA, MB, EP>(A, lda, B, ldb, M, N, K, splitk, *e, err, max_ctas, st);
@@ -431,7 +421,6 @@ extern "C" int grb_gemm_pair(int major_a, int major_b, int epi, const void* A, i
   GRB_CASE(MAJOR_K, MAJOR_K, EPI_STORE_F32)
   GRB_CASE(MAJOR_K, MAJOR_K, EPI_BIAS_GELU)
   GRB_CASE(MAJOR_K, MAJOR_K, EPI_RESID_F32)
-  GRB_CASE(MAJOR_K, MAJOR_K, EPI_CE)
   GRB_CASE(MAJOR_K, MAJOR_MN, EPI_STORE_BF16)
   GRB_CASE(MAJOR_K, MAJOR_MN, EPI_STORE_F32)
   GRB_CASE(MAJOR_K, MAJOR_MN, EPI_GELU_BWD)

@@ -27,6 +27,7 @@
 #include "ptx.cuh"
 #include "tmap.h"
 #include "scan.h"
+#include "launch.h"
 
 namespace grb {
 
@@ -263,6 +264,8 @@ scan_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   }
   if constexpr (CL) cluster_sync();             // every CTA's barriers are ready for the others' aggregates
   else __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x == 0) {
     if (CL) { ex.arm(0); ex.arm(1); }
     for (int r = 0; r < Sh::STAGES && r < rounds; ++r) issue(r);
@@ -412,6 +415,8 @@ scan_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   }
   if constexpr (CL) cluster_sync();             // every CTA's barriers are ready for the others' aggregates
   else __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x == 0) {
     if (CL) { ex.arm(0); ex.arm(1); }
     for (int r = 0; r < Sh::STAGES && r < rounds; ++r) issue(r);
@@ -582,17 +587,7 @@ static int launch_scan(Kern kern, size_t& granted, int groups, int B, int S, voi
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
     granted = smem;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(groups * S, B);
-  cfg.blockDim = dim3(Sh::THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = reinterpret_cast<cudaStream_t>(st);
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = S > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? 0 : -5;
+  return launch_pdl(kern, dim3(groups * S, B), Sh::THREADS, smem, reinterpret_cast<cudaStream_t>(st), S, args...);
 }
 
 struct ScanIo {                       // inputs of both directions (h and g are the backward's)

@@ -17,8 +17,9 @@ from ._lib import (EPI_BIAS_GELU, EPI_CE, EPI_GELU_BWD, EPI_RED_F32, EPI_RED_SCA
                    EPI_STORE_F32, MAJOR_K, MAJOR_MN, EpiArgs)
 
 LAUNCHES = 0  # number of kernels of this library launched by this process
-# Which tcgen05 GEMM kernel runs: "auto" picks the CTA-pair kernel (cta_group::2, 256x256 tiles per pair of SMs)
-# when the problem has enough tiles to fill the machine and the single-CTA kernel (128x256 tiles) otherwise.
+# Which tcgen05 GEMM kernel runs: "auto" takes the one that grb_gemm_plan estimates to be faster, CTA pairs (cta_group::2,
+# 256x256 tiles per pair of SMs) or single CTAs (128x128 tiles, K split over a cluster); "2cta" / "1cta" force one (the
+# cross-entropy epilogue exists in the single-CTA kernel only).
 GEMM_MODE = os.environ.get("GRB_GEMM", "auto")
 
 
@@ -98,10 +99,18 @@ def gemm(major_a: int, major_b: int, epi: int, a: torch.Tensor, b: torch.Tensor,
         e.gather_lo, e.gather_hi, e.gather_dst = int(glo), int(ghi), int(gdst)
     lda = int(lda if lda is not None else a.stride(0))
     ldb = int(ldb if ldb is not None else b.stride(0))
-    pair_tiles = -(-M // 256) * -(-N // 256) * max(1, splitk)
-    if splitk < 0:      # stream-K (accumulating epilogues): work is dealt in k-block runs, so count those
-        pair_tiles = -(-M // 256) * -(-N // 256) * -(-K // 64) // 8
-    use_pair = GEMM_MODE == "2cta" or (GEMM_MODE == "auto" and pair_tiles >= 48)
+    if GEMM_MODE == "2cta" and epi != EPI_CE:
+        split = 0
+    elif GEMM_MODE == "auto" and (sidecopy or gather is not None):
+        # only the pair kernel copies while it computes
+        split = 0 if -(-M // 256) * -(-N // 256) >= 48 else 1
+    else:
+        split = L.lib().grb_gemm_plan(epi, M, N, K, splitk)
+        if GEMM_MODE == "1cta":
+            split = splitk if splitk > 1 else max(split, 1)
+    use_pair = split == 0
+    if not use_pair:
+        splitk = split
     if sidecopy and not use_pair:
         copy_segments(sidecopy)          # the single-CTA kernel has no copy warps
     if gather is not None and not use_pair:
