@@ -5,7 +5,14 @@
 // Filtering follows the reference's `sample` (generate.py:30-79): logits / T; top-k keeps every entry with fewer
 // than k strictly larger ones (ties at the k-th value stay); top-p sorts descending and drops an entry when the
 // probability mass in front of it already exceeds p (the first entry that crosses the threshold stays).
+//
+// What bounds it is one block's chain of latencies between two decode steps, so the sums over the vocabulary run four wide
+// (the mass in front of an entry) or as a shuffle scan (the CDF), the blocks of a cluster meet to advance the step
+// counter where a second kernel did, and the launch overlaps the drain of the step before (launch.h).  With the logits
+// cleared inside the step, a token of a 320 x 12 model takes 171.1 us (174.1 before), 512 x 32 466 (472), 2048 x 20 652.6 (661.6),
+// eight sequences of it 866 (875).
 #include "sample.h"
+#include "launch.h"
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
@@ -23,6 +30,22 @@ __device__ __forceinline__ float block_max(float v, float* sh) {
   for (int w = 1; w < 8; ++w) r = fmaxf(r, sh[w]);
   __syncthreads();
   return r;
+}
+// Sum over this thread's and all earlier ones.
+__device__ __forceinline__ float block_prefix(float v, float* sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
+  }
+  if (lane == 31) sh[warp] = v;
+  __syncthreads();
+  float before = 0.f;
+#pragma unroll
+  for (int w = 0; w < 7; ++w) before += w < warp ? sh[w] : 0.f;
+  __syncthreads();
+  return before + v;
 }
 __device__ __forceinline__ float block_sum(float v, float* sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -49,11 +72,14 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
 __global__ void __launch_bounds__(256) sample_kernel(const float* __restrict__ logits, int V, float temperature, int top_k,
                                                      float top_p, const float* __restrict__ u_in, unsigned long long seed,
                                                      long long* step_counter, unsigned char* tok_out, long long* history,
-                                                     int hist_len, float* probs_out) {
-  __shared__ float l[256], p[256], red[8];
+                                                     int hist_len, float* probs_out, int blocks_meet) {
+  __shared__ __align__(16) float l[256], p[256];
+  __shared__ float red[8];
   __shared__ int winner;
   const int i = threadIdx.x, b = blockIdx.x;
   const bool in = i < V;
+  pdl_trigger();
+  pdl_wait();
   const long long step = step_counter ? step_counter[0] : 0;
   if (step_counter) seed += static_cast<unsigned long long>(step_counter[1]);   // per-generation seed, set by the host
   float li = in ? logits[static_cast<size_t>(b) * V + i] : -CUDART_INF_F;
@@ -75,8 +101,12 @@ __global__ void __launch_bounds__(256) sample_kernel(const float* __restrict__ l
     __syncthreads();
     bool keep = in;
     if (top_k > 0 && top_k < V) {
-      int greater = 0;
-      for (int j = 0; j < V; ++j) greater += l[j] > li ? 1 : 0;
+      int greater = 0;                         // entries V .. 255 hold -inf and no mass
+#pragma unroll 8
+      for (int j = 0; j < 256; j += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(l + j);
+        greater += (t.x > li) + (t.y > li) + (t.z > li) + (t.w > li);
+      }
       keep = keep && greater < top_k;
     }
     const float m = block_max(keep ? li : -CUDART_INF_F, red);
@@ -87,21 +117,23 @@ __global__ void __launch_bounds__(256) sample_kernel(const float* __restrict__ l
     __syncthreads();
     if (top_p > 0.f) {
       // probability mass sorted in front of entry i (descending value, lower index first among equals)
-      float before = 0.f;
-      for (int j = 0; j < V; ++j)
-        if (l[j] > li || (l[j] == li && j < i)) before += p[j];
-      if (before > top_p) pi = 0.f;
+      float4 front = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+      for (int j = 0; j < 256; j += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(l + j), m = *reinterpret_cast<const float4*>(p + j);
+        if (t.x > li || (t.x == li && j < i)) front.x += m.x;
+        if (t.y > li || (t.y == li && j + 1 < i)) front.y += m.y;
+        if (t.z > li || (t.z == li && j + 2 < i)) front.z += m.z;
+        if (t.w > li || (t.w == li && j + 3 < i)) front.w += m.w;
+      }
+      if ((front.x + front.y) + (front.z + front.w) > top_p) pi = 0.f;
     }
     const float tot2 = block_sum(pi, red);
     pi /= tot2;
-    __syncthreads();
-    p[i] = pi;
-    __syncthreads();
     if (probs_out && in) probs_out[static_cast<size_t>(b) * V + i] = pi;
     // inverse CDF in index order: the token is the first index whose running sum exceeds u
     const float u = u_in ? u_in[b] : uniform01(seed, static_cast<unsigned long long>(step), b);
-    float run = 0.f;
-    for (int j = 0; j <= i && j < V; ++j) run += p[j];
+    const float run = block_prefix(pi, red);
     if (i == 0) winner = 256;
     __syncthreads();
     if (in && pi > 0.f && run > u) atomicMin(&winner, i);
@@ -118,6 +150,10 @@ __global__ void __launch_bounds__(256) sample_kernel(const float* __restrict__ l
     tok_out[b] = static_cast<unsigned char>(tok);
     if (history && step < hist_len) history[static_cast<size_t>(b) * hist_len + step] = tok;
   }
+  if (blocks_meet) {                          // one cluster: every block has read the counter
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (b == 0 && i == 0) *step_counter = step + 1;
+  }
 }
 
 __global__ void bump_kernel(long long* counter) { *counter += 1; }
@@ -130,9 +166,12 @@ extern "C" int grb_sample(const float* logits, int B, int V, float temperature, 
                           float* probs_out, void* stream) {
   if (B < 1 || V < 1 || V > 256 || !logits || !tok_out || temperature < 0.f) return -50;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  grb::sample_kernel<<<B, 256, 0, st>>>(logits, V, temperature, top_k, top_p, u_in, seed,
-                                        reinterpret_cast<long long*>(step_counter), tok_out,
-                                        reinterpret_cast<long long*>(history), hist_len, probs_out);
-  if (step_counter) grb::bump_kernel<<<1, 1, 0, st>>>(reinterpret_cast<long long*>(step_counter));
+  const int meet = step_counter && B <= 8;      // 8: the largest portable cluster
+  const unsigned long long sd = seed;
+  const int rc = grb::launch_pdl(grb::sample_kernel, dim3(B), 256, 0, st, meet ? B : 1, logits, V, temperature, top_k, top_p, u_in, sd,
+                                 reinterpret_cast<long long*>(step_counter), reinterpret_cast<unsigned char*>(tok_out),
+                                 reinterpret_cast<long long*>(history), hist_len, probs_out, meet);
+  if (rc) return rc;
+  if (step_counter && !meet) grb::bump_kernel<<<1, 1, 0, st>>>(reinterpret_cast<long long*>(step_counter));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -104,11 +104,11 @@ class Decoder:
         eng = self.engine
         ix, eps, sms, ov = eng._idx, eng.eps, eng._sms, self.overlap
         K.embed_fwd(self.tok, 1, eng._p(ix["emb"]), self.x)
-        self.logits.zero_()
         for i, lx in enumerate(ix["layers"]):
             K.decode_tc(K.IN_NORM, self.x, eng._w(lx["wg"]), self.ku, vec=eng._p(lx["n1"]), zero=self.a, eps=eps, sms=sms,
                         overlap=ov)
-            K.decode_tc(K.IN_GATE, self.ku, eng._w(lx["wo"]), self.x, state=self.h[i], state_out=self.hn, sms=sms, overlap=ov)
+            K.decode_tc(K.IN_GATE, self.ku, eng._w(lx["wo"]), self.x, state=self.h[i], state_out=self.hn,
+                        zero=self.logits if i == 0 else None, sms=sms, overlap=ov)
             K.decode_tc(K.IN_NORM, self.x, eng._w(lx["w1"]), self.a, vec=eng._p(lx["n2"]), zero=self.ku,
                         copy=(self.h[i], self.hn), eps=eps, sms=sms, overlap=ov)
             K.decode_tc(K.IN_GELU, self.a, eng._w(lx["w2"]), self.x, vec=eng._p(lx["b1"]), out_bias=eng._p(lx["b2"]), sms=sms,
