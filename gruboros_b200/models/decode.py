@@ -210,7 +210,7 @@ class Decoder:
         for _ in range(n):
             if graph is not None:
                 graph.replay()
-                K.LAUNCHES += self.launches_per_step + 2
+                K.LAUNCHES += self.launches_per_step + 1
             else:
                 body()
             if on_token is not None:
