@@ -353,13 +353,22 @@ class FusedEngine:
         units.append((f.offsets[ix["emb"]], end(ix["emb"])))
         return units
 
+    def _beside(self, bufs: _Buffers):
+        """The stream for the weight gradients of a recorded backward pass, or None to leave them in line."""
+        # Beside the chain of dgrads they fill the SMs that it leaves idle: 512 x 6, batch 2 x 256 twice 1586 -> 1419 us, 320 x 12,
+        # 3 x 778 1767 -> 1623, 1024 x 85, eight chunks of 2047 199.2 -> 188.7 ms.  Dgrads of four waves and more (16376 x 2048)
+        # leave none: 200.2 ms in line, 201.1 beside.
+        if -(-bufs.M // 256) * -(-self.D // 256) >= 2 * self._sms:
+            return None
+        return torch.cuda.Stream(device=self.device)
+
     def _backward(self, bufs: _Buffers, unit_done=None) -> None:
         """Gradients of the last training forward on `bufs`, accumulated into the flat fp32 gradient buffer.
         `unit_done(j)` is called as soon as every gradient of unit j (see unit_ranges) has been launched."""
         self._check_backward(bufs)
         n0 = K.LAUNCHES
         if unit_done is None and self._recordable():
-            bufs.recorder.run(self._key("backward"), lambda: self._launch_backward(bufs), self.device)
+            bufs.recorder.run(self._key("backward"), lambda: self._launch_backward(bufs, beside=self._beside(bufs)), self.device)
         else:
             self._launch_backward(bufs, unit_done)
         self._gen += 1          # activations are consumed
@@ -371,8 +380,25 @@ class FusedEngine:
         if self.grad_sink is None and self.store is None:
             self.flat.reclaim_discarded_grads()     # gradients the caller dropped (p.grad = None) start from zero
 
-    def _launch_backward(self, bufs: _Buffers, unit_done=None) -> None:
+    def _launch_backward(self, bufs: _Buffers, unit_done=None, beside=None) -> None:
+        """``beside``: a stream for the weight gradients, which nothing in this pass waits for but the reuse of their inputs."""
         B, T, M = bufs.B, bufs.T, bufs.M
+        main = torch.cuda.current_stream()
+
+        def wgrad(dy16, x16, i, splitk):
+            if beside is None:
+                self._wgrad(dy16, x16, i, splitk)
+                return None
+            beside.wait_event(main.record_event())
+            with torch.cuda.stream(beside):
+                self._wgrad(dy16, x16, i, splitk)
+                return beside.record_event()
+
+        def reuse(read):            # the buffer that this weight gradient reads is written next
+            if read is not None:
+                main.wait_event(read)
+
+        r_da1 = r_dku = None
         D, Di, Fh, V = self.D, self.Di, self.F, self.V
         ix = self._idx
         sms = self._sms
@@ -386,7 +412,7 @@ class FusedEngine:
         # head.  Every gradient that flows into the consumer of a folded norm already carries that norm's rstd
         # (d logits from the cross-entropy epilogue, d(k,u) from the scan, d(pre-activation) from the GELU' epilogue),
         # so wgrad and dgrad run on the saved unnormalised operand and the norm's backward takes the `prescaled` form.
-        self._wgrad(bufs.dlogits, bufs.xwf, ix["logits"], sk(V, D))
+        wgrad(bufs.dlogits, bufs.xwf, ix["logits"], sk(V, D))
         K.linear_dgrad(bufs.dlogits, self._w(ix["logits"]), bufs.dy16,
                        **(pg.prefetch("bwd", self.depth) if pg is not None else {}))
         last = ix["layers"][-1]
@@ -397,24 +423,28 @@ class FusedEngine:
             lx = ix["layers"][i]
             x_in, x_mid = bufs.xs[2 * i], bufs.xs[2 * i + 1]
             # feed-forward: x_out = x_mid + gelu(RMSNorm(x_mid) W1^T + b1) W2^T + b2
-            self._wgrad(bufs.dres16, bufs.f1[i], lx["w2"], sk(D, Fh))
+            r_dres = wgrad(bufs.dres16, bufs.f1[i], lx["w2"], sk(D, Fh))
+            reuse(r_da1)
             K.linear_dgrad(bufs.dres16, self._w(lx["w2"]), bufs.da1, epi=K.EPI_GELU_BWD, aux=bufs.g1[i],
                            colsum=self._g(lx["b1"]), rowscale=bufs.rstd2[i],
                            **(pg.prefetch("bwd", i) if pg is not None else {}))
-            self._wgrad(bufs.da1, bufs.xw2[i], lx["w1"], sk(Fh, D))
+            r_da1 = wgrad(bufs.da1, bufs.xw2[i], lx["w1"], sk(Fh, D))
             K.linear_dgrad(bufs.da1, self._w(lx["w1"]), bufs.dy16)
+            reuse(r_dres)
             K.rmsnorm_bwd(bufs.dy16, x_mid, bufs.rstd2[i], self._p(lx["n2"]), dres_a, dres_b, bufs.dres16,
                           self._g(lx["n2"]), None, prescaled=True)
             # minGRU: x_mid = x_in + scan(RMSNorm(x_in) Wg^T) Wo^T
-            self._wgrad(bufs.dres16, bufs.h[i], lx["wo"], sk(D, Di))
+            r_dres = wgrad(bufs.dres16, bufs.h[i], lx["wo"], sk(D, Di))
             K.linear_dgrad(bufs.dres16, self._w(lx["wo"]), bufs.dh)
             ku3 = bufs.ku[i].view(B, T, 2 * Di)
             dku3 = bufs.dku.view(B, T, 2 * Di)
+            reuse(r_dku)
             K.scan_bwd(ku3[..., Di:], ku3[..., :Di], bufs.h[i].view(B, T, Di), bufs.dh.view(B, T, Di),
                        dku3[..., Di:], dku3[..., :Di], h0=bufs.h0[i] if bufs.h0_valid else None, rowscale=bufs.rstd1[i])
-            self._wgrad(bufs.dku, bufs.xw1[i], lx["wg"], sk(2 * Di, D))
+            r_dku = wgrad(bufs.dku, bufs.xw1[i], lx["wg"], sk(2 * Di, D))
             K.linear_dgrad(bufs.dku, self._w(lx["wg"]), bufs.dy16)
             prev_b2 = self._g(ix["layers"][i - 1]["b2"]) if i > 0 else None
+            reuse(r_dres)
             K.rmsnorm_bwd(bufs.dy16, x_in, bufs.rstd1[i], self._p(lx["n1"]), dres_b, dres_a, bufs.dres16,
                           self._g(lx["n1"]), prev_b2, prescaled=True)
             if unit_done is not None:
@@ -422,9 +452,11 @@ class FusedEngine:
                     unit_done(0)                    # head: its last gradient (final-norm weight) came before this layer
                 unit_done(self.depth - i)
         # embedding: dE[v] += sum over rows with token v of dres  ==  onehot^T dres
-        self._wgrad(bufs.onehot, bufs.dres16, ix["emb"], sk(V, D))
+        wgrad(bufs.onehot, bufs.dres16, ix["emb"], sk(V, D))
         if unit_done is not None:
             unit_done(self.depth + 1)
+        if beside is not None:
+            main.wait_stream(beside)
 
     # ----------------------------------------------------------- public API
     @staticmethod
@@ -489,7 +521,14 @@ class FusedEngine:
         def body():
             self._launch_forward(bufs, bufs.tokens, True, alpha)
             main, side = torch.cuda.current_stream(), self._side_stream()
-            self._launch_backward(bufs, lambda j: stepper.unit_done(j, main, side))
+            beside = self._beside(bufs)
+
+            def unit_done(j):
+                if beside is not None:
+                    side.wait_stream(beside)
+                stepper.unit_done(j, main, side)
+
+            self._launch_backward(bufs, unit_done, beside)
             stepper.join(main, side)
 
         bufs.recorder.run(self._key("train", alpha, *stepper.addresses()), body, self.device)
